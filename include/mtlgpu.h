@@ -356,9 +356,12 @@ mtlgpu_status mtlgpu_pc_sweep_f32(mtlgpu_pc* P, int which, const float* d_in, fl
 mtlgpu_status mtlgpu_pc_set_jacobi_sweeps(mtlgpu_pc* P, int iters);
 /* Diagnostics (no counterpart in the reference): how the solves of P apply
  * factor `which` in precision `prec`: *kind = 0 level-ordered sync-free sweep,
- * 1 partitioned sweep (contexts created with MTLGPU_SWEEP=part, where the
- * partition fits shared memory), 2 Jacobi iterations
- * (mtlgpu_pc_set_jacobi_sweeps). */
+ * 1 partitioned sweep (factors with narrow levels and short rows, and contexts
+ * created with MTLGPU_SWEEP=part, where the partition fits shared memory),
+ * 2 Jacobi iterations (mtlgpu_pc_set_jacobi_sweeps).  A factor with the
+ * pattern of a grid stencil is swept along its grid lines, in tiles of lines
+ * handed over in shared memory, unless the context was created with
+ * MTLGPU_SWEEP=part or =ticket; it reports the kind its levels would choose. */
 mtlgpu_status mtlgpu_pc_sweep_kind(const mtlgpu_pc* P, int which, int prec, int* kind);
 /* Factor sizes and level counts: nnz of the factor as the reference stores it
  * (L of IC(0) includes the diagonal, L of ILU(0) does not). */

@@ -221,7 +221,7 @@ mtlgpu_status compute_levels(Ctx* ctx, int n, const int32_t* d_rp, const int32_t
   return MTLGPU_OK;
 }
 
-void free_sweep_plan(Ctx* ctx, SweepPlan* p) {
+void free_sweep_arrays(Ctx* ctx, SweepPlan* p) {
   part_plan_free(ctx, p);
   dfree(ctx, p->d_rp);
   dfree(ctx, p->d_ci);
@@ -232,8 +232,13 @@ void free_sweep_plan(Ctx* ctx, SweepPlan* p) {
   dfree(ctx, p->d_row_of);
   dfree(ctx, p->d_task_ptr);
   dfree(ctx, p->d_level_ptr);
-  dfree(ctx, p->d_level);
   dfree(ctx, p->d_ticket);
+}
+
+void free_sweep_plan(Ctx* ctx, SweepPlan* p) {
+  free_sweep_arrays(ctx, p);
+  line_plan_free(ctx, p);
+  dfree(ctx, p->d_level);
   *p = SweepPlan();
 }
 

@@ -552,6 +552,7 @@ mtlgpu_status mtlgpu_pc_sweep(mtlgpu_pc* P, int which, const double* in, double*
   if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0) || in == out)
     return MTLGPU_INVALID_ARG;
   const SweepPlan& S = which == MTLGPU_LOWER ? P->lower : P->upper;
+  MTLGPU_TRY(pc_ensure_sweeps(P, MTLGPU_FP64));
   MTLGPU_TRY(sweep_launch<double>(P->A->ctx, S, in, out, false, nullptr));
   return take_device_error(P->A->ctx);
 }
@@ -561,6 +562,7 @@ mtlgpu_status mtlgpu_pc_sweep_f32(mtlgpu_pc* P, int which, const float* in, floa
       P->prec != MTLGPU_FP32)
     return MTLGPU_INVALID_ARG;
   const SweepPlan& S = which == MTLGPU_LOWER ? P->lower : P->upper;
+  MTLGPU_TRY(pc_ensure_sweeps(P, MTLGPU_FP32));
   MTLGPU_TRY(sweep_launch<float>(P->A->ctx, S, in, out, false, nullptr));
   return take_device_error(P->A->ctx);
 }
@@ -580,6 +582,10 @@ mtlgpu_status mtlgpu_pc_sweep_kind(const mtlgpu_pc* P, int which, int prec, int*
   const int pi = prec == MTLGPU_FP32 ? 1 : 0;
   if (P->jacobi_iters > 0)
     *kind = 2;
+  else if (S.line) {
+    MTLGPU_TRY(pc_ensure_levels(const_cast<mtlgpu_pc*>(P), which));
+    *kind = part_sweep_suits(S) ? 1 : 0;
+  }
   else
     *kind = (S.part && S.part->prec[pi].ready) ? 1 : 0;
   return MTLGPU_OK;
@@ -588,7 +594,10 @@ mtlgpu_status mtlgpu_pc_sweep_kind(const mtlgpu_pc* P, int which, int prec, int*
 mtlgpu_status mtlgpu_pc_factor_info(const mtlgpu_pc* P, int which, int* nnz, int* n_levels) {
   if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0)) return MTLGPU_INVALID_ARG;
   if (nnz) *nnz = which == MTLGPU_LOWER ? P->nnz_L : P->nnz_U;
-  if (n_levels) *n_levels = which == MTLGPU_LOWER ? P->lower.n_levels : P->upper.n_levels;
+  if (n_levels) {
+    MTLGPU_TRY(pc_ensure_levels(const_cast<mtlgpu_pc*>(P), which));
+    *n_levels = which == MTLGPU_LOWER ? P->lower.n_levels : P->upper.n_levels;
+  }
   return MTLGPU_OK;
 }
 
@@ -621,6 +630,7 @@ mtlgpu_status mtlgpu_pc_get_levels(const mtlgpu_pc* P, int which, int32_t* lev) 
     return MTLGPU_INVALID_ARG;
   Ctx* c = P->A->ctx;
   const SweepPlan& S = which == MTLGPU_LOWER ? P->lower : P->upper;
+  MTLGPU_TRY(pc_ensure_levels(const_cast<mtlgpu_pc*>(P), which));
   if (P->n)
     MTLGPU_TRY_CUDA(c, cudaMemcpyAsync(lev, S.d_level, sizeof(int32_t) * P->n,
                                        cudaMemcpyDeviceToHost, c->stream));

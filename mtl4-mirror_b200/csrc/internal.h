@@ -140,11 +140,14 @@ struct PartPlan {
   } prec[2];
 };
 
+struct LinePlan;  // grid-line form of a sweep (line_sweep.cu)
+
 // One triangular sweep, stored in processing (level) order.
 // Row t of the plan is original row row_of[t]; its off-diagonal entries are
 // ci/val[rp[t] .. rp[t+1]); dinv[t] is its (inverted) diagonal, absent for a
 // unit diagonal.  Tasks never cross a level boundary: task k covers plan rows
-// [task_ptr[k], task_ptr[k+1]).
+// [task_ptr[k], task_ptr[k+1]).  A factor with a grid-line form has only that
+// (and, once asked for, its levels).
 struct SweepPlan {
   int n = 0, nnz_off = 0, n_levels = 0, n_tasks = 0;
   int group = 4;                   // lanes per row
@@ -162,6 +165,7 @@ struct SweepPlan {
   int32_t* d_level = nullptr;      // level of each ORIGINAL row
   unsigned* d_ticket = nullptr;    // [0] = task ticket, [1] = finished warps
   PartPlan* part = nullptr;        // partitioned form, when built and fitting
+  LinePlan* line = nullptr;        // grid-line form (line_sweep.cu), for stencil factors
 };
 
 struct Pc {
@@ -265,12 +269,28 @@ mtlgpu_status fill_sentinel(Ctx* ctx, T* p, int n);
 // capture; without a usable plan (disabled, or a part that does not fit
 // shared memory) S->part stays null and sweeps use sweep_kernel.
 mtlgpu_status part_plan_build(Ctx* ctx, SweepPlan* S, bool with_fp32);
+bool part_sweep_suits(const SweepPlan& S);  // narrow levels and short rows
 void part_plan_free(Ctx* ctx, SweepPlan* S);
 void part_plan_free_one(Ctx* ctx, PartPlan* PP, int prec);
 template <typename T>
 bool part_sweep_ready(const SweepPlan& S, const T* out);
 template <typename T>
 mtlgpu_status part_sweep_launch(Ctx* ctx, const SweepPlan& S, const T* in, T* out,
+                                const int* skip);
+
+// Sweeps along grid lines (line_sweep.cu), for factors with a grid stencil's
+// pattern.  line_plan_detect and line_plan_fill run outside stream capture;
+// the records are made before the first exact sweep (pc_ensure_sweeps).
+mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* S, const SweepPlan* like, const int32_t* d_rp,
+                               const int32_t* d_ci);
+mtlgpu_status line_plan_fill(Ctx* ctx, SweepPlan* S, int prec, const int32_t* d_rp,
+                             const int32_t* d_ci, const double* d_v, bool round);
+mtlgpu_status line_ic0_inverse(Ctx* ctx, SweepPlan* L, const int32_t* d_rp, const int32_t* d_ci,
+                               const double* d_a, double* d_inv, int* d_pivot);
+void line_plan_free(Ctx* ctx, SweepPlan* S);
+bool line_records_ready(const SweepPlan& S, int prec);
+template <typename T>
+mtlgpu_status line_sweep_launch(Ctx* ctx, const SweepPlan& S, const T* in, T* out,
                                 const int* skip);
 
 // SELL-32 layouts (sell.cu).  diag_pos: 0 = every entry kept (a matrix, or
@@ -320,6 +340,7 @@ mtlgpu_status build_sweep_plan(Ctx* ctx, int n, const int32_t* d_rp, const int32
                                const double* d_v, bool lower, bool unit_diag, bool diag_last,
                                SweepPlan* plan);
 void free_sweep_plan(Ctx* ctx, SweepPlan* plan);
+void free_sweep_arrays(Ctx* ctx, SweepPlan* plan);  // all but the levels and the grid-line form
 mtlgpu_status sweep_plan_make_fp32(Ctx* ctx, SweepPlan* plan);
 mtlgpu_status compute_levels(Ctx* ctx, int n, const int32_t* d_rp, const int32_t* d_ci,
                              bool lower, int32_t* d_level, int* n_levels);
@@ -332,6 +353,8 @@ mtlgpu_status csr_transpose(Ctx* ctx, int n_rows, int n_cols, int nnz, const int
 mtlgpu_status pc_build(Pc* P);
 void pc_release(Pc* P);
 mtlgpu_status pc_ensure_adjoint(Pc* P);
+mtlgpu_status pc_ensure_sweeps(Pc* P, int prec);    // exact sweeps ready (before any capture)
+mtlgpu_status pc_ensure_levels(Pc* P, int which);
 template <typename T>
 mtlgpu_status pc_apply_t(Pc* P, const T* r, T* z, bool adjoint, const int* skip,
                          bool prefilled_tmp, bool prefilled_out, double* rho_out = nullptr);

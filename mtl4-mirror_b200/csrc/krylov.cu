@@ -777,6 +777,8 @@ constexpr int prec_of(float*) { return MTLGPU_FP32; }
 template <typename T>
 mtlgpu_status get_workspace(Csr* A, Pc* P, int method, Workspace<T>** out) {
   const int prec = prec_of((T*)nullptr);
+  // the sweeps' plans are made outside the recorded graphs
+  if (method >= 0 && uses_sweeps(P)) MTLGPU_TRY(pc_ensure_sweeps(P, prec));
   for (auto& e : A->workspaces)
     if (e.P == P && e.method == method && e.prec == prec) {
       *out = static_cast<Workspace<T>*>(e.ws);

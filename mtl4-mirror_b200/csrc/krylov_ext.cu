@@ -1362,6 +1362,8 @@ mtlgpu_status solve_krylov_impl(int method, Csr* A, Pc* L, Pc* R, int param, dou
     res->norm_r0 = prm->norm_r0 < 0 ? 0.0 : prm->norm_r0;
     return MTLGPU_OK;
   }
+  for (Pc* P : {L, R})  // sweep plans are made outside stream capture
+    if (P && P->jacobi_iters == 0) MTLGPU_TRY(pc_ensure_sweeps(P, MTLGPU_FP64));
   XWork* W = nullptr;
   MTLGPU_TRY(create_xwork(A, L, R, method, param, &W));
   Rec r{W, ctx};

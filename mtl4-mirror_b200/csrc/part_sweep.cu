@@ -673,20 +673,23 @@ bool part_plan_host(const PartInput& in, HostPart* out) {
   return true;
 }
 
-// Built at preconditioner creation (outside any stream capture).
+bool part_sweep_suits(const SweepPlan& S) {
+  return S.n_levels > 0 && S.n / S.n_levels <= kAutoRowsPerLevel &&
+         (long long)S.nnz_off * 2 <= 5ll * S.n;
+}
+
+// Built at preconditioner creation (outside any stream capture), for factors
+// that have no grid-line form.
 mtlgpu_status part_plan_build(Ctx* ctx, SweepPlan* S, bool with_fp32) {
   part_plan_free(ctx, S);
   const int n = S->n;
-  if (n == 0 || ctx->part_sweeps == 0) return MTLGPU_OK;
+  if (n == 0 || ctx->part_sweeps == 0 || S->line) return MTLGPU_OK;
   // automatic choice: the partitioned sweep where levels are narrow (few rows
   // per level, long dependency chains) and factor rows short (2-D 5-point
   // grids, where it measured 16 % faster); the level-ordered ticket sweep
   // where levels are wide (3-D grids) or rows long (27-point factors: 5.7 ms
   // partitioned against under 1 ms for the ticket sweep at 48^3)
-  if (ctx->part_sweeps == 2 &&
-      (S->n_levels == 0 || n / S->n_levels > kAutoRowsPerLevel ||
-       (long long)S->nnz_off * 2 > 5ll * n))
-    return MTLGPU_OK;
+  if (ctx->part_sweeps == 2 && !part_sweep_suits(*S)) return MTLGPU_OK;
 
   // host copies of the level-ordered plan
   std::vector<int32_t> lp(S->n_levels + 1), row_of(n), rp(n + 1), ci(S->nnz_off);

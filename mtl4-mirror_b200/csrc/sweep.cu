@@ -133,11 +133,13 @@ mtlgpu_status sweep_launch(Ctx* ctx, const SweepPlan& P, const T* in, T* out, bo
   if (P.n == 0) return MTLGPU_OK;
   const T* val = PlanVals<T>::val(P);
   const T* dinv = PlanVals<T>::dinv(P);
-  if ((P.nnz_off > 0 && !val) || (!P.unit_diag && !dinv)) return MTLGPU_INVALID_ARG;
+  const bool line = line_records_ready(P, sizeof(T) == 8 ? 0 : 1);
+  if (!line && ((P.nnz_off > 0 && !val) || (!P.unit_diag && !dinv))) return MTLGPU_INVALID_ARG;
   if (!prefilled) {
     MTLGPU_TRY(fill_sentinel<T>(ctx, out, P.n));
     ctx->launches++;
   }
+  if (line) return line_sweep_launch<T>(ctx, P, in, out, skip);
   if (part_sweep_ready<T>(P, out)) return part_sweep_launch<T>(ctx, P, in, out, skip);
   ctx->launches++;
   const int R = 32 / P.group;

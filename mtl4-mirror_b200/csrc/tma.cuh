@@ -25,6 +25,9 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
 
 // mbarrier helpers (shared::cta, 64-bit barrier objects).
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
