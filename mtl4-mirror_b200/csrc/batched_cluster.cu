@@ -814,8 +814,8 @@ mtlgpu_status batch_work_build(Csr* A, Pc* P, int count, const int32_t* h_off, d
     a.dinv32 = P->d_inv_diag32;
   } else if (P && (P->kind == MTLGPU_PC_IC0 || P->kind == MTLGPU_PC_ILU0)) {
     a.pc = 2;
-    a.L = P->jac_lower;
-    a.U = P->jac_upper;
+    a.L = P->jac_lower.grid ? P->slice_lower : P->jac_lower;
+    a.U = P->jac_upper.grid ? P->slice_upper : P->jac_upper;
     a.jac_k = P->jacobi_iters;
   }
   a.b = d_b;
@@ -888,6 +888,8 @@ mtlgpu_status solve_batched_cluster(Csr* A, Pc* P, int count, const int32_t* h_o
   if (refine && P && P->kind != MTLGPU_PC_IDENTITY && P->prec != MTLGPU_FP32)
     return MTLGPU_INVALID_ARG;
   if (refine) MTLGPU_TRY(csr_ensure_fp32(A));
+  if (P && (P->kind == MTLGPU_PC_IC0 || P->kind == MTLGPU_PC_ILU0))
+    MTLGPU_TRY(pc_jacobi_slices(P));
   const unsigned long long hsh = hash_offsets(h_off, count);
   BatchWork* w = static_cast<BatchWork*>(A->batch_work);
   const int pk = P ? P->kind : -1, jk = P ? P->jacobi_iters : 0;

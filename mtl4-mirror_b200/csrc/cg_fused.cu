@@ -35,6 +35,7 @@
 #include <cstring>
 
 #include "device.cuh"
+#include "grid_rows.cuh"
 #include "internal.h"
 #include "solver_state.cuh"
 
@@ -54,6 +55,18 @@ template <typename T>
 constexpr int min_blocks_a() { return sizeof(T) == 4 ? 6 : 4; }
 template <typename T>
 constexpr int min_blocks_c() { return sizeof(T) == 4 ? 6 : 5; }
+
+// The same on the grid layout (grid_rows.cuh).  K_A by W and type: the 128^3
+// mixed solve took 24.1 ms with 6 blocks (5: 24.6, 4: 25.4, 3: 27.1, 8: 26.2),
+// its FP64 counterpart with two Jacobi iterations 27.3 with 5 (4: 27.5, 6: 28.8,
+// 3: 28.9), the 96^3 27-point BiCGSTAB solve 11.1 with 5 (4: 11.4, 3: 11.5, 6:
+// 11.3).  K_C 4: 26.7 us in FP32 and 38.4 in FP64 at 128^3 (5: 34 / 51, 3: 33 /
+// 39, 6: 30 / 43).
+template <typename T>
+constexpr int grid_blocks_a(int W) { return W == 13 || sizeof(T) == 8 ? 5 : 6; }
+constexpr int kGridBlocksC = 4;
+template <typename T>
+constexpr int grid_blocks_t() { return sizeof(T) == 4 ? 5 : 4; }
 
 int rows_grid(Ctx* ctx, long long n, int per_sm) {
   const long long need = (n + kBlock - 1) / kBlock;
@@ -89,6 +102,41 @@ __device__ __forceinline__ int sell_col(const int32_t* __restrict__ col,
     return d == -32768 ? -1 : row + d;
   }
   return in ? __ldlu(col + o) : -1;
+}
+
+// K_A's scalars, by the last block to arrive: r'.r' (or s.s), the iteration
+// count and the termination test.
+template <typename T, bool BICG>
+__device__ __forceinline__ void lupd_finish(typename AccOf<T, 1>::type acc, double gamma,
+                                            SolverState* st, void* partials, unsigned* counter) {
+  typedef typename AccOf<T, 1>::type R;
+  R bs = block_reduce(acc);
+  R* parts = reinterpret_cast<R*>(partials);
+  if (publish_partial(bs, parts, blockIdx.x, counter, gridDim.x)) {
+    R tot = reduce_partials(parts, gridDim.x);
+    if (threadIdx.x == 0) {
+      if (BICG) {
+        if (gamma == 0.0) {
+          st->status = MTLGPU_BREAKDOWN;
+          st->done = 1;
+          st->skip2 = 1;
+        } else {
+          st->alpha_1 = st->rho / gamma;  // alpha
+          st->ss = tot.value(0);
+          if (iter_finished(st, sqrt(st->ss))) {
+            st->half_exit = 1;
+            st->skip2 = 1;
+          }
+        }
+      } else {
+        const double rr = tot.value(0);
+        st->iter++;
+        st->rho_1 = st->rho;
+        st->rr = rr;
+        if (iter_finished(st, sqrt(fabs(rr)))) st->done = 1;
+      }
+    }
+  }
 }
 
 // K_A.  The Jacobi pass is jacobi_pass_kernel's (same chunking, same
@@ -141,33 +189,42 @@ __global__ void __launch_bounds__(kBlock, min_blocks_a<T>())
     if (SCALE) res *= dr;
     out[row] = res;
   }
-  R bs = block_reduce(acc_rr);
-  R* parts = reinterpret_cast<R*>(partials);
-  if (publish_partial(bs, parts, blockIdx.x, counter, gridDim.x)) {
-    R tot = reduce_partials(parts, gridDim.x);
-    if (threadIdx.x == 0) {
-      if (BICG) {
-        if (gamma == 0.0) {
-          st->status = MTLGPU_BREAKDOWN;
-          st->done = 1;
-          st->skip2 = 1;
-        } else {
-          st->alpha_1 = st->rho / gamma;  // alpha
-          st->ss = tot.value(0);
-          if (iter_finished(st, sqrt(st->ss))) {
-            st->half_exit = 1;
-            st->skip2 = 1;
-          }
-        }
-      } else {
-        const double rr = tot.value(0);
-        st->iter++;
-        st->rho_1 = st->rho;
-        st->rr = rr;
-        if (iter_finished(st, sqrt(fabs(rr)))) st->done = 1;
-      }
+  lupd_finish<T, BICG>(acc_rr, gamma, st, partials, counter);
+}
+
+// K_A on the grid layout (grid_rows.cuh).
+template <typename T, bool SCALE, int W, bool BICG>
+__global__ void __launch_bounds__(kBlock, grid_blocks_a<T>(W))
+    cg_lupd_grid_kernel(const __grid_constant__ GridView A, const T* __restrict__ val,
+                        const T* __restrict__ dinv, T* __restrict__ x, const T* __restrict__ p,
+                        const T* __restrict__ r, const T* __restrict__ q, T* __restrict__ r_next,
+                        T* __restrict__ out, SolverState* st, void* partials, unsigned* counter) {
+  if (st->done) return;
+  typedef typename AccOf<T, 1>::type R;
+  const double gamma = st->gamma;
+  const T alpha = (T)(BICG ? st->rho / gamma : st->rho / st->alpha_1);
+  R acc_rr = R::zero();
+  for (long long r0 = gtid() & ~31ll; r0 < A.n; r0 += gstride()) {
+    const int row = (int)r0 + (threadIdx.x & 31), at = min(row, A.n - 1);
+    const GridRow<T, W> g(A, row);
+    const T rr0 = __ldg(r + at), q0 = __ldg(q + at);
+    const T p0 = BICG ? T(0) : __ldg(p + at), x0 = BICG ? T(0) : x[at];
+    const T dr = SCALE ? __ldg(dinv + at) : T(1);
+    T acc = T(0);
+    struct RQ { T r, q; };
+    g.template entries<grid_chunk(W)>(val, [&](int c) { return RQ{__ldg(r + c), __ldg(q + c)}; },
+                                      [&](T a, RQ e) { acc += a * next_r(e.r, e.q, alpha); });
+    if (row < A.n) {
+      const T rv = next_r(rr0, q0, alpha);
+      r_next[row] = rv;
+      if (!BICG) x[row] = fma_t(alpha, p0, x0);
+      acc_rr.add_prod(0, rv, rv);
+      T res = rv - acc;
+      if (SCALE) res *= dr;
+      out[row] = res;
     }
   }
+  lupd_finish<T, BICG>(acc_rr, gamma, st, partials, counter);
 }
 
 // K_C.  The product is spmv_sell's (stored order, products and sums rounded
@@ -217,6 +274,44 @@ __global__ void __launch_bounds__(kBlock, min_blocks_c<T>())
     }
     q[row] = sum;
     acc_pq.add_prod(0, pr, sum);
+  }
+  R bs = block_reduce(acc_pq);
+  R* parts = reinterpret_cast<R*>(partials);
+  if (publish_partial(bs, parts, blockIdx.x, counter, gridDim.x)) {
+    R tot = reduce_partials(parts, gridDim.x);
+    if (threadIdx.x == 0) *pq = tot.value(0);
+  }
+}
+
+// K_C on the grid layout.
+template <typename T, int W, bool FIRST>
+__global__ void __launch_bounds__(kBlock, kGridBlocksC)
+    cg_pspmv_grid_kernel(const __grid_constant__ GridView A, const T* __restrict__ val,
+                         const T* __restrict__ z, const T* __restrict__ p, T* __restrict__ p_next,
+                         T* __restrict__ q, const int* skip, const double* num,
+                         const double* den, double beta_value, double* pq, void* partials,
+                         unsigned* counter) {
+  if (skip && *skip) return;
+  typedef typename AccOf<T, 1>::type R;
+  const T beta = FIRST ? T(0) : (T)(num ? *num / *den : beta_value);
+  R acc_pq = R::zero();
+  for (long long r0 = gtid() & ~31ll; r0 < A.n; r0 += gstride()) {
+    const int row = (int)r0 + (threadIdx.x & 31), at = min(row, A.n - 1);
+    const GridRow<T, W> g(A, row);
+    const T z0 = __ldg(z + at), p0 = FIRST ? T(0) : __ldg(p + at);
+    T sum = T(0);
+    struct ZP { T z, p; };
+    g.template entries<grid_chunk(W)>(
+        val, [&](int c) { return ZP{__ldg(z + c), FIRST ? T(0) : __ldg(p + c)}; },
+        [&](T a, ZP e) {
+          sum = add_rn(sum, mul_rn(a, FIRST ? e.z : next_p(e.z, e.p, beta)));
+        });
+    if (row < A.n) {
+      const T pr = FIRST ? z0 : next_p(z0, p0, beta);
+      p_next[row] = pr;
+      q[row] = sum;
+      acc_pq.add_prod(0, pr, sum);
+    }
   }
   R bs = block_reduce(acc_pq);
   R* parts = reinterpret_cast<R*>(partials);
@@ -304,6 +399,39 @@ __global__ void __launch_bounds__(kBlock, min_blocks_c<T>())
   }
 }
 
+// t = A shat and the two dots on the grid layout.
+template <typename T, int W>
+__global__ void __launch_bounds__(kBlock, grid_blocks_t<T>())
+    bicg_tprod_grid_kernel(const __grid_constant__ GridView A, const T* __restrict__ val,
+                           const T* __restrict__ shat, const T* __restrict__ s,
+                           T* __restrict__ t, SolverState* st, void* partials, unsigned* counter) {
+  if (st->done || st->skip2) return;
+  typedef typename AccOf<T, 2>::type R;
+  R acc = R::zero();
+  for (long long r0 = gtid() & ~31ll; r0 < A.n; r0 += gstride()) {
+    const int row = (int)r0 + (threadIdx.x & 31);
+    const GridRow<T, W> g(A, row);
+    const T s0 = __ldg(s + min(row, A.n - 1));
+    T sum = T(0);
+    g.template entries<grid_chunk(W)>(val, [&](int c) { return __ldg(shat + c); },
+                                      [&](T a, T x) { sum = add_rn(sum, mul_rn(a, x)); });
+    if (row < A.n) {
+      t[row] = sum;
+      acc.add_prod(0, sum, s0);
+      acc.add_prod(1, sum, sum);
+    }
+  }
+  R bs = block_reduce(acc);
+  R* parts = reinterpret_cast<R*>(partials);
+  if (publish_partial(bs, parts, blockIdx.x, counter, gridDim.x)) {
+    R tot = reduce_partials(parts, gridDim.x);
+    if (threadIdx.x == 0) {
+      st->ts = tot.value(0);
+      st->tt = tot.value(1);
+    }
+  }
+}
+
 struct BetaSrc {
   const int* skip;
   const double *num, *den;  // beta = *num / *den, or value when num is null
@@ -314,8 +442,19 @@ struct BetaSrc {
 template <typename T, bool FIRST>
 void launch_pspmv(Ctx* ctx, const Sell& S, const T* val, const T* z, const T* p, T* p_next, T* q,
                   const BetaSrc& b) {
-  const int grid = rows_grid(ctx, S.n, min_blocks_c<T>());
   unsigned* ctr = counter_slot(ctx, 11);
+  if (S.grid) {
+#define MTLGPU_PG(W)                                                                         \
+  cg_pspmv_grid_kernel<T, W, FIRST>                                                          \
+      <<<grid_blocks(ctx, S.n, kBlock, kGridBlocksC), kBlock, 0, ctx->stream>>>(             \
+          grid_view(S), val, z, p, p_next, q, b.skip, b.num, b.den, b.value, b.pq,           \
+          ctx->d_partials, ctr)
+    MTLGPU_BY_MATRIX(S.W, MTLGPU_PG)
+#undef MTLGPU_PG
+    ctx->launches++;
+    return;
+  }
+  const int grid = rows_grid(ctx, S.n, min_blocks_c<T>());
   if (product_d16(S))
     cg_pspmv_kernel<T, 8, true, FIRST><<<grid, kBlock, 0, ctx->stream>>>(
         S.n, S.d_slice_ptr, S.d_col, S.d_dcol, val, z, p, p_next, q, b.skip, b.num, b.den,
@@ -350,6 +489,17 @@ void launch_lupd_c(Ctx* ctx, const Sell& L, const T* val, const T* dinv, T* x, c
 template <typename T, bool SCALE, bool BICG>
 void launch_lupd(Ctx* ctx, const Sell& L, const T* val, const T* dinv, T* x, const T* p,
                  const T* r, const T* q, T* r_next, T* out, SolverState* st) {
+  if (L.grid) {
+#define MTLGPU_LG(W)                                                                         \
+  cg_lupd_grid_kernel<T, SCALE, W, BICG>                                                     \
+      <<<grid_blocks(ctx, L.n, kBlock, grid_blocks_a<T>(W)), kBlock, 0, ctx->stream>>>(         \
+          grid_view(L), val, dinv, x, p, r, q, r_next, out, st, ctx->d_partials,             \
+          counter_slot(ctx, 10))
+    MTLGPU_BY_TRIANGLE(L.W, MTLGPU_LG)
+#undef MTLGPU_LG
+    ctx->launches++;
+    return;
+  }
   if (L.max_width <= 4)
     launch_lupd_c<T, SCALE, 4, BICG>(ctx, L, val, dinv, x, p, r, q, r_next, out, st);
   else
@@ -395,9 +545,9 @@ bool cg_fused_eligible(Csr* A, Pc* P, int prec) {
     if (!std::strcmp(e, "0")) return false;
   if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0) || P->jacobi_iters <= 0)
     return false;
-  if (A->n_rows == 0 || A->spmv_kernel != 2 || !A->sell.d_slice_ptr) return false;
+  if (A->n_rows == 0 || A->spmv_kernel != 2 || !A->sell.ready()) return false;
   const Sell& L = P->jac_lower;
-  if (!L.d_slice_ptr || (!L.unit_diag && !L.col_scaled)) return false;
+  if (!L.ready() || (!L.unit_diag && !L.col_scaled)) return false;
   if (prec == MTLGPU_FP32)
     return A->sell.d_val32 && L.d_val32 && P->jac_upper.d_val32 && P->d_tmp32 && P->d_jtmp32 &&
            (L.unit_diag || L.d_dinv32);
@@ -446,7 +596,15 @@ mtlgpu_status bicg_t_product(Csr* A, SolverState* st, const T* shat, const T* s,
   const T* val = Vals<T>::val(S);
   const int grid = rows_grid(ctx, S.n, min_blocks_c<T>());
   unsigned* ctr = counter_slot(ctx, 12);
-  if (product_d16(S))
+#define MTLGPU_TG(W)                                                                         \
+  bicg_tprod_grid_kernel<T, W>                                                               \
+      <<<grid_blocks(ctx, S.n, kBlock, grid_blocks_t<T>()), kBlock, 0, ctx->stream>>>(       \
+          grid_view(S), val, shat, s, t, st, ctx->d_partials, ctr)
+  if (S.grid) {
+    MTLGPU_BY_MATRIX(S.W, MTLGPU_TG)
+#undef MTLGPU_TG
+  }
+  else if (product_d16(S))
     bicg_tprod_kernel<T, 8, true><<<grid, kBlock, 0, ctx->stream>>>(
         S.n, S.d_slice_ptr, S.d_col, S.d_dcol, val, shat, s, t, st, ctx->d_partials, ctr);
   else
@@ -469,7 +627,7 @@ mtlgpu_status cg_direction_product(Csr* A, const T* z, double beta, const T* p, 
                                    double* d_pq) {
   Ctx* ctx = A->ctx;
   if (A->n_rows == 0) return MTLGPU_OK;
-  if (A->spmv_kernel != 2 || !A->sell.d_slice_ptr) return MTLGPU_NOT_SUPPORTED;
+  if (A->spmv_kernel != 2 || !A->sell.ready()) return MTLGPU_NOT_SUPPORTED;
   const T* val = Vals<T>::val(A->sell);
   if (!val) return MTLGPU_INVALID_ARG;
   const BetaSrc b{nullptr, nullptr, nullptr, beta, d_pq};

@@ -459,8 +459,9 @@ mtlgpu_status build_ic0(Pc* P) {
   MTLGPU_TRY(dalloc(ctx, &d_pivot, 1));
   MTLGPU_TRY_CUDA(ctx, cudaMemsetAsync(d_pivot, 0, sizeof(int), ctx->stream));
   // A grid stencil's factor: the inverses along grid lines, and no
-  // level-ordered plans (line_sweep.cu).  128^3: the whole set-up 7.5 -> 2.9
-  // ms, of which the level analyses and sorts were 4.
+  // level-ordered or partitioned plans (line_sweep.cu).  The whole set-up: 128^3
+  // 7.3 -> 1.2 ms, 64^3 1.8 -> 0.6 ms (level analyses, sorts, plan copies), 1000^2
+  // 1,206 -> 1.4 ms (the partitions made on the host).
   set_plan_shape(&P->lower, n, nu - n, true, false);
   set_plan_shape(&P->upper, n, nu - n, false, false);
   MTLGPU_TRY(line_plan_detect(ctx, &P->upper, nullptr, P->d_Urp, P->d_Uci));
@@ -725,6 +726,8 @@ void pc_release(Pc* P) {
   free_sweep_plan(ctx, &P->adj_upper);
   sell_free(ctx, &P->jac_lower);
   sell_free(ctx, &P->jac_upper);
+  sell_free(ctx, &P->slice_lower);
+  sell_free(ctx, &P->slice_upper);
   dfree(ctx, P->d_jtmp);
   dfree(ctx, P->d_jtmp32);
 }
@@ -737,18 +740,34 @@ mtlgpu_status pc_set_jacobi(Pc* P, int iters) {
   if (iters < 0) return MTLGPU_INVALID_ARG;
   if (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0) return iters ? MTLGPU_INVALID_ARG : MTLGPU_OK;
   Ctx* ctx = P->A->ctx;
-  if (iters > 0 && !P->jac_lower.d_slice_ptr && P->n > 0) {
+  if (iters > 0 && !P->jac_lower.ready() && P->n > 0) {
     const bool f32 = P->prec == MTLGPU_FP32;
     const int lower_diag = P->kind == MTLGPU_PC_IC0 ? 2 : 0;
     MTLGPU_TRY(sell_build(ctx, P->n, P->d_Lrp, P->d_Lci, P->d_Lv, lower_diag, true, f32, f32,
-                          true, &P->jac_lower));
-    MTLGPU_TRY(sell_build(ctx, P->n, P->d_Urp, P->d_Uci, P->d_Uv, 1, true, f32, f32, true,
+                          true, true, &P->jac_lower));
+    MTLGPU_TRY(sell_build(ctx, P->n, P->d_Urp, P->d_Uci, P->d_Uv, 1, true, f32, f32, true, true,
                           &P->jac_upper));
     MTLGPU_TRY(dalloc(ctx, &P->d_jtmp, P->n));
     if (f32) MTLGPU_TRY(dalloc(ctx, &P->d_jtmp32, P->n));
     MTLGPU_TRY(take_device_error(ctx));
   }
   P->jacobi_iters = iters;
+  return MTLGPU_OK;
+}
+
+// The batched kernel walks its systems' rows in SELL-32 slices: makes them
+// where the factors took the grid layout.
+mtlgpu_status pc_jacobi_slices(Pc* P) {
+  if (P->jacobi_iters == 0 || P->n == 0) return MTLGPU_OK;
+  Ctx* ctx = P->A->ctx;
+  const bool f32 = P->prec == MTLGPU_FP32;
+  if (P->jac_lower.grid && !P->slice_lower.ready())
+    MTLGPU_TRY(sell_build(ctx, P->n, P->d_Lrp, P->d_Lci, P->d_Lv,
+                          P->kind == MTLGPU_PC_IC0 ? 2 : 0, true, f32, f32, true, false,
+                          &P->slice_lower));
+  if (P->jac_upper.grid && !P->slice_upper.ready())
+    MTLGPU_TRY(sell_build(ctx, P->n, P->d_Urp, P->d_Uci, P->d_Uv, 1, true, f32, f32, true, false,
+                          &P->slice_upper));
   return MTLGPU_OK;
 }
 

@@ -79,6 +79,14 @@ struct Sell {
   float* d_val32 = nullptr;
   double* d_dinv = nullptr;
   float* d_dinv32 = nullptr;
+  // Grid layout instead of the slices (grid_rows.cuh), for stencil matrices:
+  // W offsets for the whole matrix, a mask of them per row, values by offset.
+  // d_val / d_val32 then hold that layout's values, d_slice_ptr is null.
+  bool grid = false;
+  int W = 0, mask_bytes = 0;
+  int off[32] = {};
+  uint8_t* d_mask = nullptr;
+  bool ready() const { return grid || d_slice_ptr; }
 };
 
 struct Pc;
@@ -188,6 +196,7 @@ struct Pc {
   // Triangular solves as Jacobi iterations (0: exact sweeps).
   int jacobi_iters = 0;
   Sell jac_lower, jac_upper;
+  Sell slice_lower, slice_upper;   // SELL-32 slices beside a grid layout, once asked for
   double* d_jtmp = nullptr;
   float* d_jtmp32 = nullptr;
 };
@@ -297,14 +306,17 @@ mtlgpu_status line_sweep_launch(Ctx* ctx, const SweepPlan& S, const T* in, T* ou
 // a unit-diagonal factor), 1 = the first entry of each row is the diagonal,
 // 2 = the last one; the diagonal then goes to d_dinv.
 long long sell_padded_entries(int n, const int32_t* h_rp, int diag_pos);
+// grid_ok: the grid layout may be chosen.
 mtlgpu_status sell_build(Ctx* ctx, int n, const int32_t* d_rp, const int32_t* d_ci,
                          const double* d_v, int diag_pos, bool fp64, bool fp32, bool round64,
-                         bool scale_cols, Sell* J);
+                         bool scale_cols, bool grid_ok, Sell* J);
 mtlgpu_status sell_refill(Ctx* ctx, const int32_t* d_rp, const int32_t* d_ci, const double* d_v,
                           int diag_pos, Sell* J);
 mtlgpu_status sell_ensure_fp32(Ctx* ctx, const int32_t* d_rp, const int32_t* d_ci,
                                const double* d_v, int diag_pos, Sell* J);
 void sell_free(Ctx* ctx, Sell* J);
+mtlgpu_status sample_offsets(Ctx* ctx, int n, const int32_t* d_rp, const int32_t* d_ci,
+                             int diag_pos, int* off, int* count);
 
 // Jacobi-iteration triangular solves (jacobi_sweep.cu).
 template <typename T>
@@ -316,6 +328,7 @@ mtlgpu_status jacobi_solve_from(Ctx* ctx, const Sell& J, int k, int first, const
                                 T* scratch, const int* skip, const T* dot_with = nullptr,
                                 double* dot_out = nullptr);
 mtlgpu_status pc_set_jacobi(Pc* P, int iters);
+mtlgpu_status pc_jacobi_slices(Pc* P);  // the factors as SELL-32 slices (batched solves)
 
 // Preconditioned CG with Jacobi-applied IC(0)/ILU(0) in three kernels per
 // iteration (cg_fused.cu).  `st` is the solve's device SolverState.

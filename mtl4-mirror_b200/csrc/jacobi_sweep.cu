@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "device.cuh"
+#include "grid_rows.cuh"
 #include "internal.h"
 
 namespace mtlgpu {
@@ -118,6 +119,44 @@ __global__ void __launch_bounds__(kBlock, (C == 4 && sizeof(T) == 4) ? 8 : 6)
   }
 }
 
+// The same iteration on the grid layout (grid_rows.cuh).  Blocks per SM: 6 (an
+// FP32 apply at 128^3, two passes, 24.6 us; 4: 28.7, 8: 24.4), 3 for the 27-point
+// triangles (24.8; 4: 28.7, 6: 30.2).
+constexpr int grid_per_sm(int W) { return W == 13 ? 3 : 6; }
+template <typename T, bool SCALE, bool DOT, int W>
+__global__ void __launch_bounds__(kBlock, grid_per_sm(W))
+    jacobi_grid_kernel(const __grid_constant__ GridView A, const T* __restrict__ val,
+                       const T* __restrict__ dinv, const T* __restrict__ v,
+                       const T* __restrict__ in, T* __restrict__ out, const int* skip,
+                       PassDot dot) {
+  if (skip && ld_relaxed(skip)) return;
+  typedef typename AccOf<T, 1>::type R;
+  R acc_dot = R::zero();
+  for (long long r0 = gtid() & ~31ll; r0 < A.n; r0 += gstride()) {
+    const int r = (int)r0 + (threadIdx.x & 31), at = min(r, A.n - 1);
+    const GridRow<T, W> g(A, r);
+    const T vr = __ldg(v + at), dr = SCALE ? __ldg(dinv + at) : T(1);
+    const T dw = DOT ? __ldg(static_cast<const T*>(dot.with) + at) : T(0);
+    T acc = T(0);
+    g.template entries<grid_chunk(W)>(val, [&](int c) { return __ldg(in + c); },
+                                      [&](T a, T x) { acc += a * x; });
+    T res = vr - acc;
+    if (SCALE) res *= dr;
+    if (r < A.n) {
+      out[r] = res;
+      if (DOT) acc_dot.add_prod(0, dw, res);
+    }
+  }
+  if (DOT) {
+    R bs = block_reduce(acc_dot);
+    R* parts = reinterpret_cast<R*>(dot.partials);
+    if (publish_partial(bs, parts, blockIdx.x, dot.counter, gridDim.x)) {
+      R tot = reduce_partials(parts, gridDim.x);
+      if (threadIdx.x == 0) *dot.out = tot.value(0);
+    }
+  }
+}
+
 template <typename T>
 struct JVals;
 template <>
@@ -134,8 +173,22 @@ struct JVals<float> {
 // Chunk width C: 4 when no row has more than 4 off-diagonal entries (the
 // 7-point factors), else 8.
 template <typename T, bool SCALE>
-void launch2(int grid, cudaStream_t st, const Sell& J, const T* val, const T* dinv, const T* v,
+void launch2(Ctx* ctx, int grid, const Sell& J, const T* val, const T* dinv, const T* v,
              const T* in, T* out, const int* skip, const PassDot& dot) {
+  cudaStream_t st = ctx->stream;
+  if (J.grid) {
+    const int blocks = grid_blocks(ctx, J.n, kBlock, grid_per_sm(J.W));
+#define MTLGPU_JG(W)                                                                        \
+  if (dot.out)                                                                              \
+    jacobi_grid_kernel<T, SCALE, true, W><<<blocks, kBlock, 0, st>>>(grid_view(J), val, dinv, v, \
+                                                                     in, out, skip, dot);   \
+  else                                                                                      \
+    jacobi_grid_kernel<T, SCALE, false, W><<<blocks, kBlock, 0, st>>>(grid_view(J), val, dinv, v, \
+                                                                      in, out, skip, dot)
+    MTLGPU_BY_TRIANGLE(J.W, MTLGPU_JG)
+#undef MTLGPU_JG
+    return;
+  }
 #define MTLGPU_JP(DOT, C, D16)                                                          \
   jacobi_pass_kernel<T, SCALE, DOT, C, D16><<<grid, kBlock, 0, st>>>(                   \
       J.n, J.d_slice_ptr, J.d_col, J.d_dcol, val, dinv, v, in, out, skip, dot)
@@ -164,9 +217,9 @@ mtlgpu_status pass_launch(Ctx* ctx, const Sell& J, bool scale, const T* v, const
   if (!val || (scale && !dinv) || (!J.unit_diag && !J.col_scaled)) return MTLGPU_INVALID_ARG;
   const int grid = grid_rows(ctx, J.n);
   if (scale)
-    launch2<T, true>(grid, ctx->stream, J, val, dinv, v, in, out, skip, dot);
+    launch2<T, true>(ctx, grid, J, val, dinv, v, in, out, skip, dot);
   else
-    launch2<T, false>(grid, ctx->stream, J, val, dinv, v, in, out, skip, dot);
+    launch2<T, false>(ctx, grid, J, val, dinv, v, in, out, skip, dot);
   ctx->launches++;
   MTLGPU_TRY_CUDA(ctx, cudaGetLastError());
   return MTLGPU_OK;

@@ -537,37 +537,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
 // ---------------------------------------------------------------------------
 // Analysis.
 
-// Distances of the off-diagonal entries: a table of up to kMaxOff distinct
-// ones; over[0] is set when there are more.  Entries on the diagonal (stored
-// inverted diagonals) are skipped.
-__global__ void line_distances_kernel(int n, const int32_t* __restrict__ rp,
-                                      const int32_t* __restrict__ ci, int* table, int* over) {
-  __shared__ int seen[kMaxOff];
-  if (threadIdx.x < kMaxOff) seen[threadIdx.x] = 0;
-  __syncthreads();
-  for (long long r = gtid(); r < n; r += gstride()) {
-    if (ld_relaxed(over)) return;
-    for (int j = rp[r]; j < rp[r + 1]; j++) {
-      const int d = abs(ci[j] - (int)r);
-      if (d == 0) continue;
-      bool known = false;
-      for (int k = 0; k < kMaxOff; k++) known = known || ((volatile int*)seen)[k] == d;
-      if (known) continue;
-      for (int k = 0; k <= kMaxOff; k++) {
-        if (k == kMaxOff) {
-          st_relaxed(over, 1);
-          return;
-        }
-        const int old = atomicCAS(table + k, 0, d);
-        if (old == 0 || old == d) {
-          seen[k] = d;
-          break;
-        }
-      }
-    }
-  }
-}
-
 // Entry k (farthest first; k = G E: the predecessor) of row (i, j, t): whether
 // its place is in the grid, and its distance.
 __device__ __forceinline__ bool entry_of(const LineShape& S, int k, int i, int j, int t, int* d) {
@@ -797,16 +766,13 @@ mtlgpu_status line_find(Ctx* ctx, LineShape* S, const int32_t* d_rp, const int32
                         bool* found) {
   *found = false;
   const int n = S->n;
-  int h[32];                     // distances, then the overflow flag
-  MTLGPU_TRY_CUDA(ctx, cudaMemsetAsync(d_s, 0, sizeof(h), ctx->stream));
-  line_distances_kernel<<<line_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, d_rp, d_ci, d_s, d_s + 16);
-  MTLGPU_TRY_CUDA(ctx, cudaGetLastError());
-  MTLGPU_TRY_CUDA(ctx, cudaMemcpyAsync(h, d_s, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-  MTLGPU_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  int d[kMaxOff], nd = 0;
-  for (int k = 0; k < kMaxOff && h[k]; k++) d[nd++] = h[k];
+  int off[32], cnt = 0, d[kMaxOff], nd = 0;
+  MTLGPU_TRY(sample_offsets(ctx, n, d_rp, d_ci, 0, off, &cnt));
+  if (cnt > kMaxOff + 1) return MTLGPU_OK;
+  for (int k = 0; k < cnt; k++)
+    if (off[k] && nd < kMaxOff) d[nd++] = std::abs(off[k]);
   std::sort(d, d + nd, [](int x, int y) { return x > y; });
-  if (h[16] || nd < 2 || d[nd - 1] != 1) return MTLGPU_OK;
+  if (nd < 2 || d[nd - 1] != 1) return MTLGPU_OK;
   // candidates: B a distance, P a number of lines at another distance, or (two
   // dimensions) all lines in one plane
   for (int kb = nd - 2; kb >= 0; kb--) {
@@ -818,7 +784,7 @@ mtlgpu_status line_find(Ctx* ctx, LineShape* S, const int32_t* d_rp, const int32
       if (lp < 2 || lp > lines || lines % lp || !line_stencil(d, nd, B, lp, S)) continue;
       S->NI = lines / lp;
       for (S->asc = 0; S->asc < 2; S->asc++) {
-        MTLGPU_TRY(line_verify(ctx, *S, d_rp, d_ci, d_s + 16, found));
+        MTLGPU_TRY(line_verify(ctx, *S, d_rp, d_ci, d_s, found));
         if (*found) return MTLGPU_OK;
       }
     }
@@ -845,7 +811,7 @@ mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* P, const SweepPlan* like, co
   if (P->n == 0 || P->nnz_off == 0 || ctx->part_sweeps != 2 || (like && !like->line))
     return MTLGPU_OK;
   int* d_s = nullptr;
-  MTLGPU_TRY(dalloc(ctx, &d_s, 32));
+  MTLGPU_TRY(dalloc(ctx, &d_s, 1));
   LineShape S{};
   bool found = false;
   mtlgpu_status st = MTLGPU_OK;

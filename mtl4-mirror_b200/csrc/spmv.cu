@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "device.cuh"
+#include "grid_rows.cuh"
 #include "internal.h"
 #include "tma.cuh"
 
@@ -333,6 +334,29 @@ __global__ void __launch_bounds__(kBlock, 8)
   finish_epilogue(ep, acc);
 }
 
+// The product on the grid layout (grid_rows.cuh): same row sums, same bits.
+// Blocks per SM, by the 128^3 7-point product: FP64 4 (22.5 us; 5: 24.7, 6: 30.8,
+// 3: 24.6), FP32 5 (16.4; 4: 16.9, 6: 18.5).
+template <typename T>
+constexpr int grid_per_sm() { return sizeof(T) == 4 ? 5 : 4; }
+template <typename T, int W>
+__global__ void __launch_bounds__(kBlock, grid_per_sm<T>())
+    spmv_grid(const __grid_constant__ GridView A, const T* __restrict__ val,
+              const T* __restrict__ x, T* __restrict__ y, EpiParams<T> ep) {
+  if (ep.skip && ld_relaxed(ep.skip)) return;
+  typedef typename AccOf<T, 1>::type R;
+  R acc = R::zero();
+  for (long long r0 = gtid() & ~31ll; r0 < A.n; r0 += gstride()) {
+    const int r = (int)r0 + (threadIdx.x & 31);
+    const GridRow<T, W> g(A, r);
+    T sum = T(0);
+    g.template entries<grid_chunk(W)>(val, [&](int c) { return __ldg(x + c); },
+                                      [&](T a, T xv) { sum = add_rn(sum, mul_rn(a, xv)); });
+    if (r < A.n) row_epilogue(ep, r, sum, y, acc);
+  }
+  finish_epilogue(ep, acc);
+}
+
 template <typename T>
 void launch_group(int G, int grid, cudaStream_t st, int nrows, const int32_t* rows,
                   const int32_t* rp, const int32_t* ci, const T* v, const T* x, T* y,
@@ -399,7 +423,7 @@ mtlgpu_status csr_analyse(Csr* A) {
     }
     if (A->spmv_kernel == 2)
       MTLGPU_TRY(sell_build(ctx, A->n_rows, A->d_rp, A->d_ci, A->d_v, 0, true, false, false,
-                            false, &A->sell));
+                            false, A->n_rows == A->n_cols, &A->sell));
     const int cap = 32 * kStreamK;
     std::vector<int2> blk;
     blk.reserve(A->n_rows / 16 + 2);
@@ -521,6 +545,19 @@ mtlgpu_status spmv_launch(Csr* A, const T* x, T* y, const SpmvArgs& args) {
   if (A->spmv_kernel == 2) {
     const T* sv = csr_sell_values<T>(A);
     if (!sv) return MTLGPU_INVALID_ARG;
+    if (A->sell.grid) {
+      const int blocks = grid_blocks(ctx, A->n_rows, kBlock, grid_per_sm<T>());
+      ep.part_off = 0;
+      ep.part_total = blocks;
+      ep.final_launch = true;
+#define MTLGPU_SG(W) \
+  spmv_grid<T, W><<<blocks, kBlock, 0, ctx->stream>>>(grid_view(A->sell), sv, x, y, ep)
+      MTLGPU_BY_MATRIX(A->sell.W, MTLGPU_SG)
+#undef MTLGPU_SG
+      ctx->launches++;
+      MTLGPU_TRY_CUDA(ctx, cudaGetLastError());
+      return MTLGPU_OK;
+    }
     const int grid = grid_for(ctx, kBlock, A->n_rows);
     ep.part_off = 0;
     ep.part_total = grid;
@@ -601,7 +638,7 @@ mtlgpu_status csr_autotune_spmv(Csr* A, int* choice, float* ms) {
     *choice = A->spmv_kernel;
     return MTLGPU_OK;
   }
-  if (A->spmv_kernel != 2 && !A->sell.d_slice_ptr) {
+  if (A->spmv_kernel != 2 && !A->sell.ready()) {
     std::vector<int32_t> h_rp(A->n_rows + 1);
     MTLGPU_TRY_CUDA(ctx, cudaMemcpyAsync(h_rp.data(), A->d_rp, sizeof(int32_t) * (A->n_rows + 1),
                                          cudaMemcpyDeviceToHost, ctx->stream));
@@ -609,7 +646,7 @@ mtlgpu_status csr_autotune_spmv(Csr* A, int* choice, float* ms) {
     const long long padded = sell_padded_entries(A->n_rows, h_rp.data(), 0);
     if (padded <= 2ll * A->nnz && padded < (1ll << 31))
       MTLGPU_TRY(sell_build(ctx, A->n_rows, A->d_rp, A->d_ci, A->d_v, 0, true, false, false,
-                            false, &A->sell));
+                            false, A->n_rows == A->n_cols, &A->sell));
   }
   double *x = nullptr, *y = nullptr;
   MTLGPU_TRY(dalloc(ctx, &x, A->n_cols));
@@ -623,7 +660,7 @@ mtlgpu_status csr_autotune_spmv(Csr* A, int* choice, float* ms) {
   float best_ms = 1e30f;
   SpmvArgs plain;
   for (int k : {2, 0}) {
-    if (k == 2 && !A->sell.d_slice_ptr) continue;
+    if (k == 2 && !A->sell.ready()) continue;
     A->spmv_kernel = k;
     mtlgpu_status st = spmv_launch<double>(A, x, y, plain);
     cudaEventRecord(e0, ctx->stream);
@@ -645,7 +682,7 @@ mtlgpu_status csr_autotune_spmv(Csr* A, int* choice, float* ms) {
   }
   A->spmv_kernel = best;
   release_workspaces(A, nullptr);  // solver graphs captured the previous kernel
-  if (best != 2 && A->sell.d_slice_ptr) sell_free(ctx, &A->sell);
+  if (best != 2 && A->sell.ready()) sell_free(ctx, &A->sell);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   dfree(ctx, x);
