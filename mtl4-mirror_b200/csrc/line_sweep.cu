@@ -37,34 +37,44 @@
 // outside the grid, where the records hold zeros: rr - 0 * 0 leaves rr as it is,
 // bit for bit.
 //
-// What sets the time (B200, FP64; the sweep alone is ~25 us less than a call):
-// a step of a patch is ~190 cycles, the instruction latency of one warp (150 of
-// them in the fold: shuffle, then K multiplies and dependent subtracts), and a
-// tile boundary ~1.5 us of hand-off through L2.  One call of the lower sweep,
-// level-ordered / this kernel: 128^3 7-point 546 / 175 us, 96^3 27-point
-// 850 / 365 us, 512^2 5-point 1,145 / 147 us (partitioned: 850), 100^2 224 / 52
-// us.  Earlier forms of this kernel on 512^2: lanes advancing independently
-// (per-lane bounds, masks and copies) 830 us; lanes in step with tagged slots
-// polled and voted on per row 281 us; the loaders' addresses recomputed per
-// copy 292 us.  KS = 8 (E = 1) measured 190 us at 128^3.
+// What sets the time (B200): a step of a patch, and the hand-off between tiles.
+// A step is 115-120 cycles in two dimensions and FP64 (FP32 95), ~190-220 in
+// three: the chain shuffle, multiply, K dependent subtracts, multiply, and the
+// issue of the warp's ~32 instructions.  So a step's operands are read a step
+// ahead, a block's inputs are asked for during the block before, a block whose
+// lanes all have rows has no tests per row, and records lie in memory as the
+// stages have them, one bulk copy per stage: 88 instructions and 240 cycles a
+// step before that (FP64, 512^2; 377 cycles at 128^3).  A tile boundary costs
+// 1.5-2.5 us: a store to L2, a poll, the inbox, and the rest of a block on both
+// sides.  One call of the lower sweep (~25 us of it the fill and the host's wait),
+// level-ordered / before / now: 128^3 7-point 546 / 175 / 152 us (FP32 517 / 135 /
+// 123), 96^3 27-point 850 / 365 / 279, 512^2 5-point 1,145 / 147 / 109, 100^2
+// 224 / 52 / 47.  Slower: blocks of 2 steps (512^2 144, 128^3 152-181), of 8 (128^3
+// 190 with the former kernel), and a chunk counter by cp.async groups in place of
+// the stages' mbarriers (the loader then waits for each copy).  Earlier forms on
+// 512^2: lanes advancing independently 830 us; lanes in step with tagged slots
+// polled and voted on per row 281.
 //
 // A CTA's warps:
 //   compute  a thread per line: shuffles and inbox values, fold, publish.
-//   fetch    a few lanes per halo line (lines of neighbouring tiles that this
+//   fetch    several lanes per halo line (lines of neighbouring tiles that this
 //            tile depends on), one row each: poll the NaN-boxed output vector in
-//            L2 and file the values in the inboxes.  (One lane polling several
+//            L2 and file the values in the inboxes.  A poll takes ~1,000 cycles,
+//            so the lanes bound the rate of rows (two dimensions: 4 lanes 160 us
+//            at 512^2, 8 lanes 113, 16 lanes 109).  (One lane polling several
 //            rows: its loads of one cache line wait for each other, ~500 cycles
 //            each.)
-//   load     a warp per compute warp: cp.async of a block's records and
-//            right-hand sides of its 32 lines into a ring of stages, one
-//            mbarrier each, in whole cache lines.
+//   load     a warp per compute warp, per stage of KL steps: its records with one
+//            bulk copy, right-hand sides with cp.async, one mbarrier per stage.
+//            (Records too by cp.async, a block at a time: 550 cycles a block, more
+//            than the four steps they feed.)
 // A value is filed only when its reader's counter shows the ring slot free.
 // That cannot block: a warp waits for an earlier patch to be less than KS steps
 // ahead, or for a later patch or one fed by the same halo line to be within R
 // steps, and around any circle of such waits the steps lost exceed those gained
 // (R > 2 KS + the largest distance in steps between a value and its reader).
 // Records are the row's K = G E + 1 entry values, farthest first, and its
-// inverted diagonal, in x order, padded to 16 bytes.
+// inverted diagonal, padded to 16 bytes.
 //
 // Progress: tiles are claimed by an atomic ticket in an order in which every
 // dependency points to the same or an earlier tile (lines shifted by `sk` per
@@ -75,6 +85,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <initializer_list>
+#include <type_traits>
 
 #include "device.cuh"
 #include "internal.h"
@@ -111,12 +122,13 @@ template <> struct Stencil<4, 3> {  // 27-point; lines shifted by one per plane
 template <int G, int E>
 struct Shape : Stencil<G, E> {
   using S = Stencil<G, E>;
-  static constexpr int kSteps = 4;                   // steps per block
+  static constexpr int kSteps = 4;                 // steps per block
+  static constexpr int kLoad = E == 1 ? 8 : 4;     // steps per stage
   static constexpr int kRing = E == 1 ? 32 : 16;   // steps an inbox holds
   static constexpr int amax = G > 1 ? 1 : 0;       // planes a line depends on
   static constexpr int sk = G == 4 ? 1 : 0;        // lines shifted per plane
   static constexpr int hl = G == 4 ? 2 : 1;        // halo lines left of a tile
-  static constexpr int fetch = E == 1 ? 8 : 4;     // lanes per halo line
+  static constexpr int fetch = G == 1 ? 16 : E == 1 ? 8 : 4;     // lanes per halo line
   static constexpr int PJ = amax ? 8 : 32, PI = 32 / PJ;  // a warp's patch
   static constexpr int newest = E == 3 ? -1 : 0;   // place of a group's last value
   static constexpr int s1 = 1 - newest;            // skew per line
@@ -125,6 +137,11 @@ struct Shape : Stencil<G, E> {
   // exactly kSteps steps after it was made, so its slot does not wrap inside
   // a block.
   static constexpr int X = E == 1 ? kSteps - 1 : 0;
+  // step of row 0 of line (gi, gj) of a tile (three places: the step before it
+  // takes row 0 of the lines it depends on)
+  __host__ __device__ static constexpr int skew(int gi, int gj) {
+    return gj * s1 + gi * s2 + (gj / PJ + gi / PI) * X + (E == 3 ? 1 : 0);
+  }
   __host__ __device__ static constexpr int back(int g) { return newest + S::PA(g) * s2 + S::PB(g) * s1; }
   __host__ __device__ static constexpr int dist(int g) { return S::PA(g) * PJ + S::PB(g); }
   static constexpr int far = G == 4 ? 5 : 1;       // largest back(g)
@@ -138,15 +155,16 @@ struct Shape : Stencil<G, E> {
 // The stencil: G lines of dependencies (farthest first) with E places each.
 struct LineShape {
   int n, B, P, NI, G, E;
-  int mirrored, asc;             // asc: rows store their nearest entry first
+  int mirrored;                  // an upper factor: x order is reversed row order
   int a[4], b[4];
 };
 
 struct LineArgs {
-  int n, B, P, NI, TI, TJ, ntj, ntiles, mirrored;
+  int n, B, P, NI, TI, TJ, ntj, ntiles;
   int rec_bytes, stages;
-  int rec_stride, rhs_stride;   // bytes of one line's rings
-  int off_rec, off_rhs, off_bar, off_lines, off_prog, off_halo, smem;
+  int rhs_stride;               // bytes of one line's ring of right-hand sides
+  int blocks, stage;            // stages a warp's records fill, bytes of one
+  int off_rec, off_rhs, off_lines, off_prog, off_halo, off_bar, smem;
   int compute_warps, fetch_warps, steps;
 };
 
@@ -179,15 +197,15 @@ __device__ __forceinline__ void st_shared_release(unsigned a, int v) {
   asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
-// A record's values and diagonal (KR elements) from shared memory, 16 bytes
-// at a time.
+// A record's values and diagonal (KR elements) from shared memory: 16 bytes per
+// lane and 512 bytes.
 template <typename T, int KR>
 __device__ __forceinline__ void load_record(const unsigned char* s, T (&rec)[KR]) {
   constexpr int V = 16 / (int)sizeof(T);
 #pragma unroll
   for (int i = 0; i < KR; i += V) {
     T w[V];
-    ld16(reinterpret_cast<const T*>(s) + i, w);
+    ld16(reinterpret_cast<const T*>(s + i / V * 512), w);
 #pragma unroll
     for (int u = 0; u < V; u++)
       if (i + u < KR) rec[i + u] = w[u];
@@ -200,13 +218,13 @@ __host__ __device__ constexpr int rec_bytes() {
   return ((G * E + 2) * (int)sizeof(T) + 15) & ~15;
 }
 
-// ASC: rows store their nearest entry first.
+// UP: an upper factor, whose rows store their nearest entry first.
 // IC0: not a sweep but IC(0)'s inverse diagonal (itl/pc/ic_0.hpp:136-186 as
 // factor.cu has it): records hold a_mk and a_kk, and a row makes
 //     out[k] = 1 / sqrt(a_kk - sum_m (a_mk out[m])^2)     (m ascending),
 // the same dependencies with another fold; *pivot is set where that is no
 // positive finite number.
-template <typename T, int G, int E, bool ASC, bool IC0>
+template <typename T, int G, int E, bool UP, bool IC0>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     line_sweep_kernel(const __grid_constant__ LineArgs A, const unsigned char* __restrict__ recs,
                       const T* __restrict__ in, T* out, unsigned* ticket, int* err,
@@ -214,15 +232,18 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   if (skip && ld_relaxed(skip)) return;
   using S = Shape<G, E>;
   constexpr int kTs = (int)sizeof(T), K = G * E + 1, KS = S::kSteps, R = S::kRing;
+  constexpr int KL = S::kLoad;
   constexpr int kSlot = 32 * kTs;            // one step of one group of an inbox
   constexpr int kInbox = G * R * kSlot;      // one warp's inbox
+  constexpr int kRow = 32 * rec_bytes<T, G, E>(), kStage = KL * kRow;  // records of a step, a stage
   constexpr int kNever = INT32_MAX / 2;
+  constexpr int dir = UP ? -1 : 1;           // from a row to the next one in x order
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ int s_tile, s_done;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nlines = A.compute_warps * 32, npj = A.TJ / S::PJ;
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + A.off_bar);
   const unsigned sm0 = smem_u32(sm), prog = sm0 + A.off_prog, halo = sm0 + A.off_halo;
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + A.off_bar);
   int2* lines = reinterpret_cast<int2*>(sm + A.off_lines);
   if (tid == 0) {
     s_tile = (int)atomicAdd(ticket, 1u);
@@ -235,11 +256,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const int i = I0 + gi, j = J0 + gj - i * S::sk;
     return i < 0 || i >= A.NI || j < 0 || j >= A.P ? -1 : (i * A.P + j) * A.B;
   };
-  // step of row 0 of a line of the tile (three places: the step before it
-  // takes row 0 of the lines it depends on)
-  auto skew_of = [&](int gi, int gj) {
-    return gj * S::s1 + gi * S::s2 + (gj / S::PJ + gi / S::PI) * S::X + (E == 3 ? 1 : 0);
-  };
+  auto skew_of = [&](int gi, int gj) { return S::skew(gi, gj); };
   // line (gi, gj)'s thread, and its inbox address of group g
   auto thread_of = [&](int gi, int gj) {
     return (gi / S::PI * npj + gj / S::PJ) * 32 + gi % S::PI * S::PJ + gj % S::PJ;
@@ -249,7 +266,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   };
   for (int i = tid; i < A.compute_warps * kInbox / 16; i += blockDim.x)
     reinterpret_cast<int4*>(sm)[i] = make_int4(0, 0, 0, 0);
-  for (int i = tid; i < A.compute_warps * A.stages; i += blockDim.x) mbar_init(full + i, 32);
+  // a stage is there when its right-hand sides (32 lanes) and records (one) are
+  for (int i = tid; i < A.compute_warps * A.stages; i += blockDim.x) mbar_init(full + i, 33);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   for (int i = tid; i < A.compute_warps * (1 + A.fetch_warps); i += blockDim.x)
     reinterpret_cast<int*>(sm + A.off_prog)[i] = 0;  // prog, then halo
   // this thread's line
@@ -272,12 +291,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const int B = A.B, skew = skew_of(li, lj);
     // this lane's row at step s is s - lo; it has none when s - lo >= B (unsigned)
     const int lo = first < 0 ? kNever : skew;
-    const unsigned char* rec_s = sm + A.off_rec + tid * A.rec_stride;
+    const unsigned char* rec_s = sm + A.off_rec + warp * A.stages * kStage + lane * 16;
     const unsigned char* rhs_s = sm + A.off_rhs + tid * A.rhs_stride;
-    unsigned long long* bar = full + warp * A.stages;
-    const int dir = A.mirrored ? -1 : 1;
-    T* o = out + (first < 0 ? 0 : (A.mirrored ? A.n - 1 - first : first)) - (long long)dir * skew;
-    const unsigned ib = inbox_of(tid, 0);
+    const unsigned char* box_s = sm + warp * kInbox + lane * kTs;
+    T* op = out + (first < 0 ? 0 : (UP ? A.n - 1 - first : first)) - (long long)dir * skew;
     bool near[G];       // group g comes from a lane of this warp
     unsigned tgt[G];    // inbox of the line of another patch that takes this one as group g
     int tpos[G];        // slot of the value made at step 0 there
@@ -294,8 +311,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       }
     }
     // What a block waits for, one condition per lane: *cptr >= s0 + cthr.
-    unsigned cptr = 0;
-    int cthr = 0;
+    unsigned cptr = prog + warp * 4;  // no condition: its own counter, at least 0
+    int cthr = -kNever;
     {
       const int pi = warp / npj, pj = warp % npj, npi = A.TI / S::PI;
       const int r = lane % 3, up = lane < 3 ? 1 : -1;  // right, below, diagonal
@@ -315,77 +332,124 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       for (int x = 0; x < E; x++) w[g][x] = T(0);
 #pragma unroll
     for (int x = 0; x < S::far; x++) hist[x] = T(0);
-    bool dead = false;
-    for (int s0 = 0; s0 < A.steps; s0 += KS) {
-      const int blk = s0 / KS, st = blk & smask;
-      for (long long fails = 0;;) {
-        bool here = mbar_test(bar + st, (unsigned)(blk / A.stages) & 1u);
-        if (cptr) here = here && ld_shared_acquire(cptr) >= s0 + cthr;
-        if (__all_sync(0xffffffffu, here)) break;
-        if (++fails >= limit ||
-            ((fails & 1023) == 0 && __any_sync(0xffffffffu, ld_relaxed(err) != 0))) {
-          dead = true;
-          break;
-        }
-      }
-      if (dead) break;
-      __syncwarp();
-      const unsigned ring = ib + (s0 & (R - 1)) * kSlot;
-      const unsigned char* rec_b = rec_s + st * KS * rec_bytes<T, G, E>();
-      const unsigned char* rhs_b = rhs_s + st * KS * kTs;
-      T* ob = o + (long long)dir * s0;
+    // Blocks in which every lane has a row at every step: s0 in [in_lo, in_hi].
+    const int in_lo = __reduce_max_sync(0xffffffffu, lo);
+    const int in_hi = __reduce_min_sync(0xffffffffu, lo) + B - KS;
+    unsigned long long* bar = full + warp * A.stages;
+    // Whether block `s0`, whose records are in stage st, has its inputs.
+    auto gate = [&](int s0, int st, unsigned phase) {
+      const int c = ld_shared_acquire(cptr);
+      const bool m = s0 % KL != 0 || mbar_test(bar + st, phase);
+      return m & (c >= s0 + cthr);
+    };
+    // A step's operands, read a step ahead of their use: record (two of 27
+    // points in FP64 don't fit the registers), right-hand side and inbox values.
+    constexpr int RB = K * kTs > 64 ? 1 : 2;
+    T rec[RB][K + 1], rhs[2], box[2][G];
+    auto load_rec = [&](const unsigned char* p, int u) {
+      load_record<T, K + 1>(p + u * kRow, rec[u % RB]);
+    };
+    auto load = [&](const unsigned char* rp, const unsigned char* vp, const unsigned char* bp,
+                    int u) {
+      if (RB == 2) load_rec(rp, u);
+      rhs[u & 1] = *reinterpret_cast<const T*>(vp + u * kTs);
+#pragma unroll
+      for (int g = 0; g < G; g++)
+        box[u & 1][g] = *reinterpret_cast<const volatile T*>(bp + (g * R + u) * kSlot);
+    };
+    bool dead = false, ahead = false;  // ahead: this block's gate was passed in the last one
+    int st = 0;
+    unsigned phase = 0;
+    const unsigned char *rp = rec_s, *vp = rhs_s, *bp = box_s;
+    // The steps of a block; INNER: every lane has a row.
+    auto block = [&](auto inner, int s0) {
+      constexpr bool INNER = decltype(inner)::value;
+      const int t0 = s0 - lo;
       unsigned tb[G];
 #pragma unroll
       for (int g = 0; g < G; g++)  // one place: no wrap inside the block
         tb[g] = E == 1 ? tgt[g] + ((tpos[g] + s0 * kSlot) & (R * kSlot - 1)) : tgt[g];
 #pragma unroll
       for (int u = 0; u < KS; u++) {
-        const int s = s0 + u;
-        T rec[K + 1], nw[G];
-        load_record<T, K + 1>(rec_b + u * rec_bytes<T, G, E>(), rec);
-        T rr = *reinterpret_cast<const T*>(rhs_b + u * kTs);
+        bool next = false;
+        if (RB == 1) load_rec(rp, u);
+        if (u < KS - 1) {
+          load(rp, vp, bp, u + 1);
+        } else {
+          const int part = (s0 + KS) % KL;
+          if (part == 0) st = (st + 1) & smask;
+          rp = rec_s + st * kStage + part * kRow;
+          vp = rhs_s + (st * KL + part) * kTs;
+          bp = box_s + ((s0 + KS) & (R - 1)) * kSlot;
+          if (ahead) load(rp, vp, bp, 0);
+        }
+        if (u == KS - 2) {
+          const int nst = (st + 1) & smask;
+          if ((s0 + KS) % KL == 0) phase ^= nst == 0;
+          next = gate(s0 + KS, nst, phase);
+        }
+        T nw[G], rr = IC0 ? rec[u % RB][K] : rhs[u & 1];
 #pragma unroll
         for (int g = 0; g < G; g++) {
-          lds(ring + (g * R + u) * kSlot, nw[g]);
           const T x = __shfl_up_sync(0xffffffffu, hist[S::back(g) - 1], S::dist(g));
-          nw[g] = near[g] ? x : nw[g];
+          nw[g] = near[g] ? x : box[u & 1][g];
         }
-        if (IC0) rr = rec[K];
         // one entry's contribution to the row
         auto fold = [&](T a, T wv) {
           const T d = mul_rn(a, wv);
           rr = sub_rn(rr, IC0 ? mul_rn(d, d) : d);
         };
-        if (ASC) fold(rec[K - 1], hist[0]);
+        if (UP) fold(rec[u % RB][K - 1], hist[0]);
 #pragma unroll
         for (int q = 0; q < G * E; q++) {
           // farthest line first, and on it the farthest place (index E - 1);
-          // the reverse for ASC
-          const int k = ASC ? G * E - 1 - q : q, g = k / E, x = E - 1 - k % E;
-          fold(rec[k], x == 0 ? nw[g] : w[g][x > 0 ? x - 1 : 0]);
+          // the reverse for UP
+          const int k = UP ? G * E - 1 - q : q, g = k / E, x = E - 1 - k % E;
+          fold(rec[u % RB][k], x == 0 ? nw[g] : w[g][x > 0 ? x - 1 : 0]);
         }
-        if (!ASC) fold(rec[K - 1], hist[0]);
+        if (!UP) fold(rec[u % RB][K - 1], hist[0]);
         const T sum = rr;
-        rr = IC0 ? rsqrt_rn(rr) : mul_rn(rr, rec[K]);
-        const bool row = (unsigned)(s - lo) < (unsigned)B;
+        rr = IC0 ? rsqrt_rn(rr) : mul_rn(rr, rec[u % RB][K]);
+        const bool row = INNER || (unsigned)(t0 + u) < (unsigned)B;
 #pragma unroll
         for (int x = S::far - 1; x > 0; x--) hist[x] = hist[x - 1];
         hist[0] = row ? rr : T(0);
-        if (row) st_relaxed(ob + dir * u, rr);
+        if (row) st_relaxed(op + dir * u, rr);
         if (IC0 && row && (!(sum > T(0)) || !isfinite(rr)))
           atomicCAS(pivot, 0, (int)MTLGPU_ZERO_PIVOT);
 #pragma unroll
         for (int g = 0; g < G; g++) {
           if (tgt[g])
             sts(E == 1 ? tb[g] + u * kSlot
-                       : tb[g] + ((tpos[g] + s * kSlot) & (R * kSlot - 1)), hist[0]);
+                       : tb[g] + ((tpos[g] + (s0 + u) * kSlot) & (R * kSlot - 1)), hist[0]);
 #pragma unroll
           for (int x = E - 1; x > 0; x--) w[g][x] = w[g][x - 1];
           w[g][0] = nw[g];
         }
+        if (u == KS - 2) {
+          ahead = __all_sync(0xffffffffu, next) && s0 + KS < A.steps;
+          __syncwarp();
+        }
       }
+      op += dir * KS;
       __syncwarp();
       if (lane == 0) st_shared_release(prog + warp * 4, s0 + KS);
+    };
+    for (int s0 = 0; s0 < A.steps; s0 += KS) {
+      if (!ahead) {
+        for (long long fails = 0; !__all_sync(0xffffffffu, gate(s0, st, phase));) {
+          if (++fails >= limit ||
+              ((fails & 1023) == 0 && __any_sync(0xffffffffu, ld_relaxed(err) != 0))) {
+            dead = true;
+            break;
+          }
+        }
+        if (dead) break;
+        __syncwarp();
+        load(rp, vp, bp, 0);
+      }
+      if (s0 >= in_lo && s0 <= in_hi) block(std::true_type(), s0);
+      else block(std::false_type(), s0);
     }
     if (dead && lane == 0) atomicCAS(err, 0, (int)MTLGPU_TIMEOUT);
     __syncwarp();
@@ -421,8 +485,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         any = true;
       }
     }
-    const int dir = A.mirrored ? -1 : 1;
-    const T* o = out + (any ? (A.mirrored ? A.n - 1 - hfirst : hfirst) : 0);
+    const T* o = out + (any ? (UP ? A.n - 1 - hfirst : hfirst) : 0);
     // rows to file: the line's, and (three places) the zero past its end
     const int len = any ? A.B + (E == 3 ? 1 : 0) : 0, last = any ? A.B - 1 : 0;
     // the compute warps this warp's lines feed; the others never wait for it
@@ -435,12 +498,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       st_shared_release(halo + (lane * A.fetch_warps + fw) * 4, kNever);
     int t = 0;
     for (long long polls = 0; polls < limit; ++polls) {
+      const int row = t + sub;
+      T v = ld_relaxed(o + (long long)dir * min(row, last));
       int lim = len;
 #pragma unroll
       for (int g = 0; g < G; g++)
         if (cw[g] >= 0) lim = min(lim, ld_shared_acquire(prog + cw[g] * 4) + R - due[g]);
-      const int row = t + sub;
-      T v = ld_relaxed(o + (long long)dir * min(row, last));
       if (row > last) v = T(0);
       // the rows that are there, up to the first gap
       const unsigned got = __ballot_sync(0xffffffffu, row < lim && !Box<T>::is(v)) >> (lane - sub);
@@ -469,38 +532,33 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       if (__any_sync(0xffffffffu, *(volatile int*)&s_done == A.compute_warps)) break;
     }
   } else {
-    // ---- load: a warp per compute warp.  A line's block of records is kPieces
-    // 16-byte words, taken by kPl lanes; its right-hand sides by KS lanes.  The
-    // lines a lane copies for stay in registers.
-    constexpr int kPpr = rec_bytes<T, G, E>() / 16, kPieces = kPpr * KS;
-    constexpr int kPl = kPieces >= 32 ? 32 : kPieces > 16 ? 32 : kPieces > 8 ? 16 : kPieces > 4 ? 8 : 4;
-    constexpr int kRecIt = 32 / (32 / kPl), kRhsIt = KS;
-    const int cw = warp - A.compute_warps - A.fetch_warps;
-    const int c = lane % kPl, cu = c / kPpr, u = lane % KS;
+    // ---- load: a warp per compute warp.  Its records are one bulk copy per
+    // stage (they lie in memory as they do in a stage); right-hand sides of a line
+    // are taken by KL lanes, and the lines a lane copies for stay in registers.
+    constexpr int kIt = KL;
+    const int cw = warp - A.compute_warps - A.fetch_warps, u = lane % KL;
     const int2* tab = lines + cw * 32;  // (first step, row at step 0)
-    int2 rl[kRecIt], vl[kRhsIt];
+    int2 vl[kIt];
 #pragma unroll
-    for (int i = 0; i < kRecIt; i++) {
-      rl[i] = tab[lane / kPl + i * (32 / kPl)];
-      rl[i].x -= cu;
-      if (c >= kPieces) rl[i].x = kNever;
-    }
-#pragma unroll
-    for (int i = 0; i < kRhsIt; i++) {
-      vl[i] = tab[lane / KS + i * (32 / KS)];
+    for (int i = 0; i < kIt; i++) {
+      vl[i] = tab[lane / KL + i * (32 / KL)];
       vl[i].x -= u;
       vl[i].y += u;
     }
-    const int dir = A.mirrored ? -1 : 1;
-    const T* in0 = in + (A.mirrored ? A.n - 1 : 0);
-    const unsigned char* rec0 = recs + c * 16;
-    unsigned char* rec_d = sm + A.off_rec + (cw * 32 + lane / kPl) * A.rec_stride + c * 16;
-    unsigned char* rhs_d = sm + A.off_rhs + (cw * 32 + lane / KS) * A.rhs_stride + u * kTs;
+    const T* in0 = in + (UP ? A.n - 1 : 0);
+    unsigned char* rhs_d = sm + A.off_rhs + (cw * 32 + lane / KL) * A.rhs_stride + u * kTs;
+    unsigned char* rec_d = sm + A.off_rec + cw * A.stages * kStage;
+    unsigned long long* bar = full + cw * A.stages;
+    // the block of the patch's first row
+    const int b0 = skew_of(cw / npj * S::PI, cw % npj * S::PJ) / KL;
+    const unsigned char* rec0 =
+        recs + ((long long)(s_tile * A.compute_warps + cw) * A.blocks - b0) * kStage;
     long long polls = 0;
     bool stop = false;
-    for (int s0 = 0; s0 < A.steps; s0 += KS) {
-      const int st = (s0 / KS) & smask;
-      while (s0 - ld_shared_acquire(prog + cw * 4) >= A.stages * KS) {
+    int blk = 0;
+    for (; blk < A.steps / KL; blk++) {
+      const int st = blk & smask, s0 = blk * KL;
+      while (s0 + KL - ld_shared_acquire(prog + cw * 4) > A.stages * KL) {
         if (++polls >= limit || *(volatile int*)&s_done == A.compute_warps) {
           stop = true;
           break;
@@ -508,20 +566,26 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         __nanosleep(20);
       }
       if (__any_sync(0xffffffffu, stop)) break;
+      if (lane == 0) {
+        if ((unsigned)(blk - b0) < (unsigned)A.blocks) {
+          mbar_arrive_expect_tx(bar + st, kStage);
+          bulk_copy_g2s(rec_d + st * kStage, rec0 + (long long)blk * kStage, kStage, bar + st);
+        } else {
+          mbar_arrive(bar + st);
+        }
+      }
 #pragma unroll
-      for (int i = 0; i < kRecIt; i++)
-        if ((unsigned)(s0 - rl[i].x) < (unsigned)A.B)
-          cp_async16(rec_d + i * (32 / kPl) * A.rec_stride + st * KS * kPpr * 16,
-                     rec0 + (long long)(rl[i].y + s0) * (kPpr * 16));
-#pragma unroll
-      for (int i = 0; i < (IC0 ? 0 : kRhsIt); i++)
+      for (int i = 0; i < (IC0 ? 0 : kIt); i++)
         if ((unsigned)(s0 - vl[i].x) < (unsigned)A.B)
-          cp_async_ca<kTs>(rhs_d + i * (32 / KS) * A.rhs_stride + st * KS * kTs,
+          cp_async_ca<kTs>(rhs_d + i * (32 / KL) * A.rhs_stride + st * KL * kTs,
                            in0 + (long long)dir * (vl[i].y + s0));
       __syncwarp();
-      mbar_arrive_cp_async(full + cw * A.stages + st);
+      mbar_arrive_cp_async(bar + st);
     }
+    // every copy has landed before the block ends (also one that gave up)
     cp_async_wait_all();
+    for (int k = max(0, blk - A.stages); k < blk; k++)
+      mbar_wait(bar + (k & smask), (unsigned)(k / A.stages) & 1u, limit);
   }
   __syncthreads();
   if (tid == 0) {
@@ -562,7 +626,7 @@ __global__ void line_verify_kernel(LineShape S, const int32_t* __restrict__ rp,
     const int end = rp[r + 1];
     for (int kk = 0; kk < K; kk++) {
       int d;
-      if (!entry_of(S, S.asc ? K - 1 - kk : kk, i, j, t, &d)) continue;
+      if (!entry_of(S, S.mirrored ? K - 1 - kk : kk, i, j, t, &d)) continue;
       if (q < end && ci[q] == (int)r) q++;  // a diagonal stored first
       if (q >= end || (S.mirrored ? ci[q] - (int)r : (int)r - ci[q]) != d) {
         st_relaxed(bad, 1);
@@ -578,30 +642,51 @@ __global__ void line_verify_kernel(LineShape S, const int32_t* __restrict__ rp,
   }
 }
 
-// Records in x order: the entries' values farthest first (outside the grid:
-// zero), the inverted diagonal (1 for a unit diagonal), zero padding.
-// `round` gives double records the float values.
-template <typename T>
-__global__ void line_fill_kernel(LineShape S, int rec_elems, const int32_t* __restrict__ rp,
-                                 const int32_t* __restrict__ ci, const double* __restrict__ v,
-                                 bool unit, bool round, T* __restrict__ rec) {
-  const int K = S.G * S.E + 1;
-  for (long long x = gtid(); x < S.n; x += gstride()) {
-    const int r = S.mirrored ? S.n - 1 - (int)x : (int)x;
-    const int t = (int)(x % S.B), j = (int)(x / S.B % S.P), i = (int)(x / S.B / S.P);
-    T* o = rec + x * rec_elems;
+// Records: the entries' values farthest first (outside the grid: zero), the
+// inverted diagonal (1 for a unit diagonal), zero padding; row x's where the
+// sweep's stages have them: [tile][warp][stage][step][16 bytes][lane].  `round`
+// gives double records the float values.
+template <typename T, int G, int E>
+__global__ void line_fill_kernel(const __grid_constant__ LineShape L,
+                                 const __grid_constant__ LineArgs A,
+                                 const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                 const double* __restrict__ v, bool unit, bool round,
+                                 unsigned char* __restrict__ rec) {
+  using S = Shape<G, E>;
+  constexpr int K = G * E + 1, V = 16 / (int)sizeof(T), KL = S::kLoad;
+  constexpr int kPpr = rec_bytes<T, G, E>() / 16;
+  for (long long x = gtid(); x < L.n; x += gstride()) {
+    const int r = L.mirrored ? L.n - 1 - (int)x : (int)x;
+    const int t = (int)(x % L.B), j = (int)(x / L.B % L.P), i = (int)(x / L.B / L.P);
+    const int js = j + i * S::sk, gi = i % A.TI, gj = js % A.TJ;
+    const int pi = gi / S::PI, pj = gj / S::PJ, npj = A.TJ / S::PJ;
+    const int step = t + S::skew(gi, gj), b0 = S::skew(pi * S::PI, pj * S::PJ) / KL;
+    const long long warp = (long long)(i / A.TI * A.ntj + js / A.TJ) * A.compute_warps + pi * npj + pj;
+    const int lane = gi % S::PI * S::PJ + gj % S::PJ;
+    unsigned char* o = rec + (((warp * A.blocks + step / KL - b0) * KL + step % KL) * kPpr * 32 + lane) * 16;
     int q = rp[r];
-    T dia = T(1);
+    T w[kPpr * V];
+    w[K] = T(1);
     auto val = [&](int at) { return round ? (T)(float)v[at] : (T)v[at]; };
-    if (!unit) dia = val(ci[q] == r ? q : rp[r + 1] - 1);
+    if (!unit) w[K] = val(ci[q] == r ? q : rp[r + 1] - 1);
     if (!unit && ci[q] == r) q++;
+#pragma unroll
     for (int kk = 0; kk < K; kk++) {
-      const int k = S.asc ? K - 1 - kk : kk;
       int d;
-      o[k] = entry_of(S, k, i, j, t, &d) ? val(q++) : T(0);
+      if (L.mirrored)
+        w[K - 1 - kk] = entry_of(L, K - 1 - kk, i, j, t, &d) ? val(q++) : T(0);
+      else
+        w[kk] = entry_of(L, kk, i, j, t, &d) ? val(q++) : T(0);
     }
-    o[K] = dia;
-    for (int k = K + 1; k < rec_elems; k++) o[k] = T(0);
+#pragma unroll
+    for (int k = K + 1; k < kPpr * V; k++) w[k] = T(0);
+#pragma unroll
+    for (int c = 0; c < kPpr; c++) {
+      T e[V];
+#pragma unroll
+      for (int u = 0; u < V; u++) e[u] = w[c * V + u];
+      st16(reinterpret_cast<T*>(o + c * 512), e);
+    }
   }
 }
 
@@ -658,30 +743,31 @@ bool line_layout_t(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
   A->B = L.B;
   A->P = L.P;
   A->NI = L.NI;
-  A->mirrored = L.mirrored;
   A->rec_bytes = ts == 8 ? rec_bytes<double, G, E>() : rec_bytes<float, G, E>();
-  A->stages = A->rec_bytes > 64 ? 2 : 4;
-  // Three dimensions: four patches, one above the other, so that a chain
-  // crosses few tiles along the planes and 128 tiles of a 128^3 grid fill the
-  // chip (FP64 lower sweep, with the call's ~30 us: 16 x 8 lines 176 us, 8 x 16
-  // 182, 8 x 8 196, 4 x 8 221; 96^3 27-point 358 / 380 / 379 / 361).  Two
-  // dimensions: one patch (512^2: 32 lines 147 us; 64 lines 148, 128 lines 157).
-  A->TI = S::amax ? 16 : 1;
+  A->stage = S::kLoad * 32 * A->rec_bytes;
+  // Three dimensions: patches one above the other, two of them, or four where
+  // two make more tiles than the chip has SMs (a CTA per SM).  A call of the
+  // lower sweep with 8 x 8 / 16 x 8 lines (33^3, 96^3, 128^3 7-point, FP64: 55 / 60,
+  // 104 / 109, 157 / 152 us; FP32 49 / 52, 97 / 97, 136 / 124; 47^3 27-point FP32
+  // 110 / 119; 8 x 16 and 4 x 8 lines lost to both).  27 points in FP64: one patch,
+  // 47^3 124, 96^3 279 us (two: 132 / 300, four: 145 / 301).  Two dimensions: one
+  // patch.  Stages: four where they fit, else two (16 x 8 lines in FP64: the same
+  // time).
   A->TJ = S::PJ;
+  A->ntj = (L.P + (L.NI - 1) * S::sk + A->TJ - 1) / A->TJ;
+  A->TI = !S::amax ? 1 : G == 4 && ts == 8 ? 4 : 8;
+  if (A->TI == 8 && (L.NI + 7) / 8 * A->ntj > ctx->num_sms) A->TI = 16;
   const int limit = smem_limit(ctx);
-  for (;; A->TI /= 2) {
+  for (A->stages = 4;; A->stages == 4 ? A->stages = 2 : (A->stages = 4, A->TI /= 2)) {
     if (A->TI < S::PI) return false;
-    const int lines = A->TI * A->TJ, rows = A->stages * S::kSteps;
+    const int lines = A->TI * A->TJ, rows = A->stages * S::kLoad;
     const int halo = S::amax * (A->TJ + S::hl) + A->TI * S::hl;
     A->compute_warps = lines / 32;
     A->fetch_warps = (halo * S::fetch + 31) / 32;
-    // one word more than a multiple of 128 bytes per line: the lanes' accesses
-    // spread over the shared-memory banks
-    A->rec_stride = rows * A->rec_bytes + 16;
-    A->rhs_stride = (rows + 1) * ts;
+    A->rhs_stride = (rows + 1) * ts;  // the lanes' accesses spread over the banks
     int o = lines * G * S::kRing * ts;  // inboxes
     A->off_rec = o;
-    o += lines * A->rec_stride;
+    o += lines * rows * A->rec_bytes;
     A->off_rhs = o;
     o = (o + lines * A->rhs_stride + 7) & ~7;
     A->off_bar = o;
@@ -695,12 +781,13 @@ bool line_layout_t(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
     A->smem = o;
     if (o <= limit && (2 * A->compute_warps + A->fetch_warps) * 32 <= kMaxThreads) break;
   }
-  A->ntj = (L.P + (L.NI - 1) * S::sk + A->TJ - 1) / A->TJ;
   A->ntiles = A->ntj * ((L.NI + A->TI - 1) / A->TI);
   // the last line's last step makes the zero row past its end
   const int skew = (A->TJ - 1) * S::s1 + (A->TI - 1) * S::s2 +
                    (A->TJ / S::PJ + A->TI / S::PI - 2) * S::X + 1;
-  A->steps = (skew + L.B + 1 + S::kSteps - 1) / S::kSteps * S::kSteps;
+  A->steps = (skew + L.B + 1 + S::kLoad - 1) / S::kLoad * S::kLoad;
+  // from the stage of a patch's first row to that of its last
+  A->blocks = (S::kLoad - 1 + S::skew(S::PI - 1, S::PJ - 1) - S::skew(0, 0) + L.B - 1) / S::kLoad + 1;
   return true;
 }
 bool line_layout(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
@@ -716,12 +803,12 @@ using LineKernel = void (*)(const LineArgs, const unsigned char*, const T*, T*, 
 template <typename T>
 LineKernel<T> line_kernel(const LineShape& S) {
   if (S.E == 1 && S.G == 1)
-    return S.asc ? line_sweep_kernel<T, 1, 1, true, false> : line_sweep_kernel<T, 1, 1, false, false>;
+    return S.mirrored ? line_sweep_kernel<T, 1, 1, true, false> : line_sweep_kernel<T, 1, 1, false, false>;
   if (S.E == 1)
-    return S.asc ? line_sweep_kernel<T, 2, 1, true, false> : line_sweep_kernel<T, 2, 1, false, false>;
+    return S.mirrored ? line_sweep_kernel<T, 2, 1, true, false> : line_sweep_kernel<T, 2, 1, false, false>;
   if (S.G == 1)
-    return S.asc ? line_sweep_kernel<T, 1, 3, true, false> : line_sweep_kernel<T, 1, 3, false, false>;
-  return S.asc ? line_sweep_kernel<T, 4, 3, true, false> : line_sweep_kernel<T, 4, 3, false, false>;
+    return S.mirrored ? line_sweep_kernel<T, 1, 3, true, false> : line_sweep_kernel<T, 1, 3, false, false>;
+  return S.mirrored ? line_sweep_kernel<T, 4, 3, true, false> : line_sweep_kernel<T, 4, 3, false, false>;
 }
 LineKernel<double> line_ic0_kernel(const LineShape& S) {
   if (S.E == 1)
@@ -744,6 +831,21 @@ mtlgpu_status line_launch(Ctx* ctx, LineKernel<T> kernel, const LineArgs& A, con
 
 int line_grid(Ctx* ctx, int n) {
   return (int)std::min<long long>(((long long)n + kBlock - 1) / kBlock, ctx->num_sms * 8ll);
+}
+
+template <typename T>
+void line_fill_launch(Ctx* ctx, const LineShape& S, const LineArgs& A, const int32_t* rp,
+                      const int32_t* ci, const double* v, bool unit, bool round,
+                      unsigned char* rec) {
+  const int grid = line_grid(ctx, S.n);
+#define MTLGPU_LF(G, E) \
+  line_fill_kernel<T, G, E><<<grid, kBlock, 0, ctx->stream>>>(S, A, rp, ci, v, unit, round, rec)
+  if (S.E == 1) {
+    if (S.G == 1) MTLGPU_LF(1, 1); else MTLGPU_LF(2, 1);
+  } else {
+    if (S.G == 1) MTLGPU_LF(1, 3); else MTLGPU_LF(4, 3);
+  }
+#undef MTLGPU_LF
 }
 
 // Whether every row has S's entries (flag: one device int, 4 bytes of scratch).
@@ -783,10 +885,8 @@ mtlgpu_status line_find(Ctx* ctx, LineShape* S, const int32_t* d_rp, const int32
       const int lp = kp >= 0 ? round_div(d[kp], B) : lines;
       if (lp < 2 || lp > lines || lines % lp || !line_stencil(d, nd, B, lp, S)) continue;
       S->NI = lines / lp;
-      for (S->asc = 0; S->asc < 2; S->asc++) {
-        MTLGPU_TRY(line_verify(ctx, *S, d_rp, d_ci, d_s, found));
-        if (*found) return MTLGPU_OK;
-      }
+      MTLGPU_TRY(line_verify(ctx, *S, d_rp, d_ci, d_s, found));
+      if (*found) return MTLGPU_OK;
     }
   }
   return MTLGPU_OK;
@@ -818,8 +918,7 @@ mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* P, const SweepPlan* like, co
   if (like) {
     S = like->line->shape;
     S.mirrored = P->reverse;
-    for (S.asc = 0; S.asc < 2 && !found && st == MTLGPU_OK; S.asc += !found)
-      st = line_verify(ctx, S, d_rp, d_ci, d_s, &found);
+    st = line_verify(ctx, S, d_rp, d_ci, d_s, &found);
   } else {
     S.n = P->n;
     S.mirrored = P->reverse;
@@ -854,18 +953,16 @@ mtlgpu_status line_plan_fill(Ctx* ctx, SweepPlan* P, int prec, const int32_t* d_
                              const int32_t* d_ci, const double* d_v, bool round) {
   LinePlan& L = *P->line;
   const LineShape& S = L.shape;
-  const int rb = L.args[prec].rec_bytes;
+  const LineArgs& A = L.args[prec];
   unsigned char* rec = static_cast<unsigned char*>(L.d_rec[prec]);
   if (!rec) {
-    MTLGPU_TRY(dalloc(ctx, &rec, (size_t)S.n * rb));
+    MTLGPU_TRY(dalloc(ctx, &rec, (size_t)A.ntiles * A.compute_warps * A.blocks * A.stage));
     L.d_rec[prec] = rec;
   }
   if (prec)
-    line_fill_kernel<float><<<line_grid(ctx, S.n), kBlock, 0, ctx->stream>>>(
-        S, rb / 4, d_rp, d_ci, d_v, P->unit_diag, true, reinterpret_cast<float*>(rec));
+    line_fill_launch<float>(ctx, S, A, d_rp, d_ci, d_v, P->unit_diag, true, rec);
   else
-    line_fill_kernel<double><<<line_grid(ctx, S.n), kBlock, 0, ctx->stream>>>(
-        S, rb / 8, d_rp, d_ci, d_v, P->unit_diag, round, reinterpret_cast<double*>(rec));
+    line_fill_launch<double>(ctx, S, A, d_rp, d_ci, d_v, P->unit_diag, round, rec);
   MTLGPU_TRY_CUDA(ctx, cudaGetLastError());
   return MTLGPU_OK;
 }
