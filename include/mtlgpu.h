@@ -447,8 +447,10 @@ mtlgpu_status mtlgpu_solve_batched(int method, mtlgpu_csr* A, mtlgpu_pc* P, int 
 /* Tunes mtlgpu_solve_batched for these systems: times short solves (at most
  * 8 iterations, one refinement step; x is not modified) for every candidate
  * of CTAs per large system (4, 8: the thread-block cluster that runs it),
- * lanes per matrix row (4, 8, 16), and the row count below which a system is
- * solved by a single CTA (0, 8192, 32768), and keeps the fastest on A.
+ * lanes per matrix row (1, 4, 8, 16), threads per CTA (256; with 1 or 8 lanes
+ * also 512 and 1024), and the row count below which a system is solved by a
+ * single CTA (0, 8192, 32768), and keeps the fastest on A in place of the
+ * shape that follows from the systems' sizes.
  * *h_choice = 1000 * rows + 100 * CTAs + lanes.  Applies to the persistent-launch path
  * (P NULL, diagonal, or factors applied by Jacobi iterations); other
  * preconditioners return MTLGPU_NOT_SUPPORTED.  No counterpart in the

@@ -424,20 +424,20 @@ mtlgpu_status solve_batched_impl(int method, Csr* A, Pc* P, int count, const int
     if (h_off[s + 1] < h_off[s]) return MTLGPU_INVALID_ARG;
   if (batched_cluster_supported(P)) {
     MTLGPU_TRY(batch_check(A, count, h_off));
-    int cs = A->batch_cs, g = A->batch_g;
-    int small = A->batch_small;
-    // MTLGPU_BATCH_SHAPE="CTAs,lanes[,small rows]" overrides the tuned shape
+    BatchShape shape = A->batch.cs ? A->batch : batched_shape(A, count, h_off);
+    // MTLGPU_BATCH_SHAPE="CTAs,lanes[,small rows[,threads]]" overrides the shape
     // (testing); lanes 1 selects the CSR-stream SpMV
     if (const char* m = std::getenv("MTLGPU_BATCH_SHAPE")) {
-      int c2 = 0, g2 = 0, s2 = -1;
-      const int k = std::sscanf(m, "%d,%d,%d", &c2, &g2, &s2);
+      int c2 = 0, g2 = 0, s2 = -1, t2 = 256;
+      const int k = std::sscanf(m, "%d,%d,%d,%d", &c2, &g2, &s2, &t2);
       if (k >= 2 && (c2 == 1 || c2 == 2 || c2 == 4 || c2 == 8) &&
+          (t2 == 256 || t2 == 512 || t2 == 1024) &&
           (g2 == 1 || g2 == 4 || g2 == 8 || g2 == 16 || g2 == 32)) {
-        cs = c2, g = g2;
-        if (k == 3 && s2 >= 0) small = s2;
+        shape.cs = c2, shape.g = g2, shape.threads = t2;
+        if (k >= 3 && s2 >= 0) shape.small_rows = s2;
       }
     }
-    return solve_batched_cluster(A, P, count, h_off, d_x, d_b, prm, res, cs, g, small, nullptr);
+    return solve_batched_cluster(A, P, count, h_off, d_x, d_b, prm, res, shape, nullptr);
   }
   if (prm->mode == MTLGPU_SOLVE_MIXED_REFINED)
     return solve_batched_mixed(A, P, count, h_off, d_x, d_b, prm, res);
@@ -551,8 +551,8 @@ mtlgpu_status solve_batched_impl(int method, Csr* A, Pc* P, int count, const int
 }
 
 // Times the persistent kernel's candidates -- CTAs per system (the cluster
-// size), lanes per row, and the row count below which a system is solved by
-// one CTA -- on the caller's systems: a short solve each (at most 8
+// size), lanes per row, threads per CTA, and the row count below which a system
+// is solved by one CTA -- on the caller's systems: a short solve each (at most 8
 // iterations, one refinement step), from a copy of x.  Keeps the fastest on A.
 mtlgpu_status batched_autotune_impl(Csr* A, Pc* P, int count, const int32_t* h_off,
                                            const double* d_x, const double* d_b,
@@ -569,26 +569,27 @@ mtlgpu_status batched_autotune_impl(Csr* A, Pc* P, int count, const int32_t* h_o
   p.max_outer = 1;
   p.h_interrupt = nullptr;
   float best_ms = 1e30f;
-  int best_cs = A->batch_cs, best_g = A->batch_g, best_small = A->batch_small;
+  BatchShape best;
   for (int cs : {4, 8})
     for (int g : {1, 4, 8, 16})
-      for (int small : {0, 8192, 32768}) {
+      for (int small : {0, 8192, 32768})
+        for (int threads : {256, 512, 1024}) {
+        if (threads > 256 && g != 1 && g != 8) continue;  // shapes that do not exist
+        const BatchShape shape{cs, g, threads, small};
         cudaMemcpyAsync(x, d_x, sizeof(double) * A->n_rows, cudaMemcpyDeviceToDevice,
                         ctx->stream);
         float ms = 0;
-        mtlgpu_status st = solve_batched_cluster(A, P, count, h_off, x, d_b, &p, res.data(), cs,
-                                                 g, small, &ms);
+        mtlgpu_status st = solve_batched_cluster(A, P, count, h_off, x, d_b, &p, res.data(),
+                                                 shape, &ms);
         if (st != MTLGPU_OK && st != MTLGPU_MAX_ITER) {
           dfree(ctx, x);
           return st;
         }
-        if (ms < best_ms) best_ms = ms, best_cs = cs, best_g = g, best_small = small;
+        if (ms < best_ms) best_ms = ms, best = shape;
       }
-  A->batch_cs = best_cs;
-  A->batch_g = best_g;
-  A->batch_small = best_small;
+  A->batch = best;
   dfree(ctx, x);
-  if (choice) *choice = best_small * 1000 + best_cs * 100 + best_g;
+  if (choice) *choice = best.small_rows * 1000 + best.cs * 100 + best.g;
   return take_device_error(ctx);
 }
 

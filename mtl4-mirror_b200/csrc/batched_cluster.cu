@@ -30,11 +30,13 @@
 // stopping test on ||r||, the inner solve of A d = r / ||r|| in FP32 (values,
 // factors, vectors; FP64 accumulation of the dots), x += ||r|| d.
 //
-// Tunables (CS, G) are picked per matrix by mtlgpu_batched_autotune, which
-// times the candidates on the caller's systems.
+// The shape (CS, G, threads per CTA, single-CTA rows) comes from the systems'
+// sizes (batched_shape) or from mtlgpu_batched_autotune, which times the
+// candidates on the caller's systems.
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <numeric>
 #include <vector>
@@ -51,6 +53,7 @@ using namespace dev;
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kStreamChunk = 8;  // entries a lane has in flight in the stream product
 
 struct BatchState {
   double resid, norm_b;
@@ -185,7 +188,7 @@ struct CtaTeam {
 // loaded together, then 4 gathers), so a row costs one DRAM and one L2 round
 // trip per chunk rather than per entry.  Plain loads: a system's matrix is
 // read again every iteration, and the systems in flight stay in L2.
-template <typename T, int G>
+template <typename T, int G, int BT>
 __device__ __forceinline__ void spmv_rows(const int32_t* __restrict__ rp,
                                           const int32_t* __restrict__ ci,
                                           const T* __restrict__ val, const T* p, T* y, int lo,
@@ -193,7 +196,7 @@ __device__ __forceinline__ void spmv_rows(const int32_t* __restrict__ rp,
   constexpr int KK = 4;
   constexpr int R = 2;  // rows per lane group per pass, loaded together
   const int sub = threadIdx.x / G, gl = threadIdx.x % G;
-  constexpr int rows_per_pass = kThreads / G;
+  constexpr int rows_per_pass = BT / G;
   for (int base = lo; base < hi; base += R * rows_per_pass) {
     int rb[R], re[R];
 #pragma unroll
@@ -248,16 +251,16 @@ __device__ __forceinline__ void spmv_rows(const int32_t* __restrict__ rp,
 // flight instead of a lane group's few strided ones: the large systems of a
 // batch, solved by one cluster each, are bound by the bytes a CTA has in
 // flight.
-template <typename T>
+template <typename T, int BT>
 __device__ __forceinline__ void spmv_rows_stream(const int32_t* __restrict__ rp,
                                                  const int32_t* __restrict__ ci,
                                                  const T* __restrict__ val, const T* p, T* y,
                                                  int lo, int hi, double& pq, bool dot) {
-  constexpr int KS = 8;
-  constexpr int W = kThreads / 32;
-  __shared__ T sh[W][32 * KS];
+  constexpr int KS = kStreamChunk;
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  constexpr int W = BT / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* pw = sh[warp];
+  T* pw = reinterpret_cast<T*>(stream_smem) + warp * 32 * KS;
   for (int r0 = lo + warp * 32; r0 < hi; r0 += W * 32) {
     const int nr = min(32, hi - r0);
     const int row = r0 + lane;
@@ -296,26 +299,26 @@ __device__ __forceinline__ void spmv_rows_stream(const int32_t* __restrict__ rp,
 }
 
 // The SpMV of the kernel's shape: CSR-stream (G == 1) or G lanes per row.
-template <typename T, int G>
+template <typename T, int G, int BT>
 __device__ __forceinline__ void spmv_team_rows(const int32_t* __restrict__ rp,
                                                const int32_t* __restrict__ ci,
                                                const T* __restrict__ val, const T* p, T* y,
                                                int lo, int hi, double& pq, bool dot) {
   if constexpr (G == 1)
-    spmv_rows_stream<T>(rp, ci, val, p, y, lo, hi, pq, dot);
+    spmv_rows_stream<T, BT>(rp, ci, val, p, y, lo, hi, pq, dot);
   else
-    spmv_rows<T, G>(rp, ci, val, p, y, lo, hi, pq, dot);
+    spmv_rows<T, G, BT>(rp, ci, val, p, y, lo, hi, pq, dot);
 }
 
 // One Jacobi pass of a factor over rows [lo, hi): out = v - Nt in, times the
 // stored diagonal when scale (jacobi_sweep.cu).
-template <typename T>
+template <typename T, int BT>
 __device__ __forceinline__ void jacobi_rows(const Sell& F, const T* v, const T* in, T* out,
                                             bool scale, int lo, int hi) {
   const T* fv = sell_val<T>(F);
   const T* fd = sell_dinv<T>(F);
   constexpr int KK = 4;
-  for (int r = lo + threadIdx.x; r < hi; r += kThreads) {
+  for (int r = lo + threadIdx.x; r < hi; r += BT) {
     const int s = r >> 5, lane = r & 31;
     const int base = F.d_slice_ptr[s], width = (F.d_slice_ptr[s + 1] - base) >> 5;
     T acc = T(0);
@@ -343,12 +346,13 @@ __device__ __forceinline__ void jacobi_rows(const Sell& F, const T* v, const T* 
 // arithmetic and stores, so a thread keeps 4 DRAM requests per array in
 // flight instead of walking its rows one round trip at a time.
 constexpr int kU = 4;
-#define MTLGPU_ROWS_PASS(i0) for (int i0 = lo + (int)threadIdx.x; i0 < hi; i0 += kU * kThreads)
-#define MTLGPU_ROW(i0, u) ((i0) + (u) * kThreads)
+#define MTLGPU_ROWS_PASS(i0) \
+  for (int i0 = lo + (int)threadIdx.x; i0 < hi; i0 += kU * BT)
+#define MTLGPU_ROW(i0, u) ((i0) + (u) * BT)
 
 // z = M^-1 r over the CTA's rows; factors take 2 jac_k passes, each after a
 // team barrier (a pass reads other rows of the previous one).
-template <typename T, typename Team>
+template <typename T, int BT, typename Team>
 __device__ __forceinline__ void apply_pc(Team& tm, const BatchArgs& a, const BatchVecs<T>& V,
                                          int lo, int hi) {
   if (a.pc == 2) {
@@ -357,7 +361,7 @@ __device__ __forceinline__ void apply_pc(Team& tm, const BatchArgs& a, const Bat
     const T* in = V.r;
     for (int m = 0; m < k; m++) {
       T* out = ((k - 1 - m) % 2 == 0) ? V.u : V.w;
-      jacobi_rows<T>(a.L, V.r, in, out, m == k - 1 && !a.L.unit_diag, lo, hi);
+      jacobi_rows<T, BT>(a.L, V.r, in, out, m == k - 1 && !a.L.unit_diag, lo, hi);
       tm.sync();
       in = out;
     }
@@ -365,7 +369,7 @@ __device__ __forceinline__ void apply_pc(Team& tm, const BatchArgs& a, const Bat
     in = V.u;
     for (int m = 0; m < k; m++) {
       T* out = ((k - 1 - m) % 2 == 0) ? V.z : V.w;
-      jacobi_rows<T>(a.U, V.u, in, out, m == k - 1, lo, hi);
+      jacobi_rows<T, BT>(a.U, V.u, in, out, m == k - 1, lo, hi);
       if (m + 1 < k) tm.sync();
       in = out;
     }
@@ -393,7 +397,7 @@ __device__ __forceinline__ void apply_pc(Team& tm, const BatchArgs& a, const Bat
 // x with r = b - A x computed here (direct FP64).  Stops when ||r|| <= tol or
 // after max_it iterations; returns the iteration count, *resid the last
 // residual, *norm_rhs ||rhs||.
-template <typename T, int G, typename Team>
+template <typename T, int G, int BT, typename Team>
 __device__ int pcg_system(Team& tm, const BatchArgs& a,
                           const BatchVecs<T>& V, T* x, int lo, int hi, bool direct, double rtol,
                           double atol, int max_it, double* resid, double* norm_rhs,
@@ -401,12 +405,12 @@ __device__ int pcg_system(Team& tm, const BatchArgs& a,
   const T* A = vals<T>(a);
   double pq_dummy = 0;
   if (direct) {  // r = b - A x (x is the caller's initial guess)
-    spmv_team_rows<T, G>(a.rp, a.ci, A, x, V.q, lo, hi, pq_dummy, false);
+    spmv_team_rows<T, G, BT>(a.rp, a.ci, A, x, V.q, lo, hi, pq_dummy, false);
     __syncthreads();  // rows were written by their lane groups, read by thread
-    for (int i = lo + threadIdx.x; i < hi; i += kThreads) V.r[i] = (T)a.b[i] - V.q[i];
+    for (int i = lo + threadIdx.x; i < hi; i += BT) V.r[i] = (T)a.b[i] - V.q[i];
   }
   double s0[3] = {0, 0, 0};
-  for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
+  for (int i = lo + threadIdx.x; i < hi; i += BT) {
     const double ri = (double)V.r[i];
     s0[0] += ri * ri;
     if (direct) s0[1] += a.b[i] * a.b[i];
@@ -426,7 +430,7 @@ __device__ int pcg_system(Team& tm, const BatchArgs& a,
   int it = 0, fin = finished(res, it);
   double rho_1 = 0;
   while (!fin) {
-    apply_pc<T>(tm, a, V, lo, hi);
+    apply_pc<T, BT>(tm, a, V, lo, hi);
     double s1[3] = {0, 0, 0};
     MTLGPU_ROWS_PASS(i0) {
       T rv[kU], zv[kU];
@@ -458,7 +462,7 @@ __device__ int pcg_system(Team& tm, const BatchArgs& a,
     }
     tm.sync();  // p complete before the SpMV gathers it
     double s2[3] = {0, 0, 0};
-    spmv_team_rows<T, G>(a.rp, a.ci, A, V.p, V.q, lo, hi, s2[0], true);
+    spmv_team_rows<T, G, BT>(a.rp, a.ci, A, V.p, V.q, lo, hi, s2[0], true);
     tm.sum(s2);
     const T alpha = (T)(rho / s2[0]);
     double s3[3] = {0, 0, 0};
@@ -497,15 +501,15 @@ __device__ int pcg_system(Team& tm, const BatchArgs& a,
 
 // One system on rows [lo, hi) of the team: direct FP64 PCG, or FP64
 // refinement around FP32 inner PCG.
-template <typename T, int G, typename Team>
+template <typename T, int G, int BT, typename Team>
 __device__ BatchState solve_system(Team& tm, const BatchArgs& a, const BatchVecs<T>& V, int lo,
                                    int hi, int refine) {
   BatchState st{};
   if (!refine) {
     double resid = 0, nb = 0;
     int err = 0;
-    for (int i = lo + threadIdx.x; i < hi; i += kThreads) V.p[i] = T(0);
-    st.it = pcg_system<T, G>(tm, a, V, reinterpret_cast<T*>(a.x), lo, hi, true, a.rtol, a.atol,
+    for (int i = lo + threadIdx.x; i < hi; i += BT) V.p[i] = T(0);
+    st.it = pcg_system<T, G, BT>(tm, a, V, reinterpret_cast<T*>(a.x), lo, hi, true, a.rtol, a.atol,
                              a.max_iter, &resid, &nb, &err);
     st.resid = resid;
     st.norm_b = nb;
@@ -517,10 +521,10 @@ __device__ BatchState solve_system(Team& tm, const BatchArgs& a, const BatchVecs
     int total = 0, outer = 0;
     while (true) {
       double pq_dummy = 0;
-      spmv_team_rows<double, G>(a.rp, a.ci, A64, a.x, a.r64, lo, hi, pq_dummy, false);
+      spmv_team_rows<double, G, BT>(a.rp, a.ci, A64, a.x, a.r64, lo, hi, pq_dummy, false);
       __syncthreads();  // rows were written by their lane groups, read by thread
       double s0[3] = {0, 0, 0};
-      for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
+      for (int i = lo + threadIdx.x; i < hi; i += BT) {
         const double ri = a.b[i] - a.r64[i];
         a.r64[i] = ri;
         s0[0] += ri * ri;
@@ -539,7 +543,7 @@ __device__ BatchState solve_system(Team& tm, const BatchArgs& a, const BatchVecs
       const double target = nb == 0 ? a.atol : fmax(a.rtol * nb, a.atol);
       const double itol = fmax(a.inner_rtol, fmin(0.5, 0.5 * target / resid));
       const double inv = 1.0 / resid;
-      for (int i = lo + threadIdx.x; i < hi; i += kThreads) {
+      for (int i = lo + threadIdx.x; i < hi; i += BT) {
         V.r[i] = (T)(a.r64[i] * inv);
         V.d[i] = T(0);
         V.p[i] = T(0);
@@ -547,9 +551,9 @@ __device__ BatchState solve_system(Team& tm, const BatchArgs& a, const BatchVecs
       tm.sync();
       double ir = 0, in_norm = 0;
       int ierr = 0;
-      total += pcg_system<T, G>(tm, a, V, V.d, lo, hi, false, itol, 0.0,
+      total += pcg_system<T, G, BT>(tm, a, V, V.d, lo, hi, false, itol, 0.0,
                                 min(a.inner_max, a.max_iter - total), &ir, &in_norm, &ierr);
-      for (int i = lo + threadIdx.x; i < hi; i += kThreads) a.x[i] += resid * (double)V.d[i];
+      for (int i = lo + threadIdx.x; i < hi; i += BT) a.x[i] += resid * (double)V.d[i];
       outer++;
       tm.sync();  // x complete before the next residual
     }
@@ -569,8 +573,8 @@ __device__ BatchState solve_system(Team& tm, const BatchArgs& a, const BatchVecs
 // independently.
 // 4 CTAs per SM: 64 registers a thread, no spills (measured 5 % faster for
 // the FP32-refined and Jacobi-applied IC(0) solves than 3 CTAs at 80).
-template <typename T, int G>
-__global__ void __launch_bounds__(kThreads, 4)
+template <typename T, int G, int BT>
+__global__ void __launch_bounds__(BT, 1024 / BT)
     batch_cluster_kernel(BatchArgs a, BatchVecs<T> V, int refine) {
   __shared__ ClusterSum<3> cs;
   __shared__ int item;
@@ -586,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     const int slo = a.off[s], shi = a.off[s + 1], ns = shi - slo;
     const int lo = slo + (int)((long long)ns * crank / csz);
     const int hi = slo + (int)((long long)ns * (crank + 1) / csz);
-    const BatchState st = solve_system<T, G>(tm, a, V, lo, hi, refine);
+    const BatchState st = solve_system<T, G, BT>(tm, a, V, lo, hi, refine);
     if (crank == 0 && threadIdx.x == 0) a.state[s] = st;
     tm.cl.sync();  // the system's vectors are final before the cluster moves on
   }
@@ -599,7 +603,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     const int q = item;
     if (q >= n_small) break;
     const int s = a.order[a.n_large + q];
-    const BatchState st = solve_system<T, G>(tb, a, V, a.off[s], a.off[s + 1], refine);
+    const BatchState st = solve_system<T, G, BT>(tb, a, V, a.off[s], a.off[s + 1], refine);
     if (threadIdx.x == 0) a.state[s] = st;
   }
 }
@@ -618,65 +622,68 @@ __global__ void __launch_bounds__(kThreads)
   if (threadIdx.x == 0) out[s] = sqrt(acc.value(0));
 }
 
-template <typename T, int G>
-cudaError_t launch_cluster(cudaStream_t st, int cs, int clusters, const BatchArgs& a,
-                           const BatchVecs<T>& V, int refine) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(clusters * cs));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, batch_cluster_kernel<T, G>, a, V, refine);
+// Dynamic shared memory of the stream product (G == 1): FP64 products, as the
+// residuals of the refinement have them.
+size_t stream_bytes(int g, int threads) {
+  return g == 1 ? (size_t)threads * kStreamChunk * sizeof(double) : 0;
 }
 
-template <typename T, int G>
-int max_clusters(int cs) {
+// The kernel for G lanes per row and `threads` threads per CTA; 512 and 1024
+// threads exist for the shapes batched_shape chooses.
+template <typename T>
+using BatchKernel = void (*)(BatchArgs, BatchVecs<T>, int);
+template <typename T>
+BatchKernel<T> batch_kernel(int g, int threads) {
+  if (threads == 512)
+    return g == 1 ? batch_cluster_kernel<T, 1, 512> : batch_cluster_kernel<T, 8, 512>;
+  if (threads == 1024)
+    return g == 1 ? batch_cluster_kernel<T, 1, 1024> : batch_cluster_kernel<T, 8, 1024>;
+  switch (g) {
+    case 1: return batch_cluster_kernel<T, 1, 256>;
+    case 4: return batch_cluster_kernel<T, 4, 256>;
+    case 16: return batch_cluster_kernel<T, 16, 256>;
+    case 32: return batch_cluster_kernel<T, 32, 256>;
+    default: return batch_cluster_kernel<T, 8, 256>;
+  }
+}
+
+struct ClusterConfig {
+  cudaLaunchAttribute attr[1] = {};
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(cs * 256));
-  cfg.blockDim = dim3(kThreads);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  ClusterConfig(cudaStream_t st, int cs, int threads, int clusters, int g) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(clusters * cs));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = stream_bytes(g, threads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+};
+
+template <typename T>
+cudaError_t launch_cluster(cudaStream_t st, int g, int cs, int threads, int clusters,
+                           const BatchArgs& a, const BatchVecs<T>& V, int refine) {
+  ClusterConfig c(st, cs, threads, clusters, g);
+  return cudaLaunchKernelEx(&c.cfg, batch_kernel<T>(g, threads), a, V, refine);
+}
+
+// Clusters that fit the GPU at once (0: none).
+template <typename T>
+int clusters_for(int g, int cs, int threads) {
+  BatchKernel<T> k = batch_kernel<T>(g, threads);
+  ClusterConfig c(nullptr, cs, threads, 256, g);
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, batch_cluster_kernel<T, G>, &cfg) != cudaSuccess) {
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)stream_bytes(g, threads)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k, &c.cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return n;
-}
-
-template <typename T>
-cudaError_t launch_g(cudaStream_t st, int g, int cs, int clusters, const BatchArgs& a,
-                     const BatchVecs<T>& V, int refine) {
-  switch (g) {
-    case 1: return launch_cluster<T, 1>(st, cs, clusters, a, V, refine);
-    case 4: return launch_cluster<T, 4>(st, cs, clusters, a, V, refine);
-    case 16: return launch_cluster<T, 16>(st, cs, clusters, a, V, refine);
-    case 32: return launch_cluster<T, 32>(st, cs, clusters, a, V, refine);
-    default: return launch_cluster<T, 8>(st, cs, clusters, a, V, refine);
-  }
-}
-
-template <typename T>
-int clusters_for(int g, int cs) {
-  switch (g) {
-    case 1: return max_clusters<T, 1>(cs);
-    case 4: return max_clusters<T, 4>(cs);
-    case 16: return max_clusters<T, 16>(cs);
-    case 32: return max_clusters<T, 32>(cs);
-    default: return max_clusters<T, 8>(cs);
-  }
 }
 
 }  // namespace
@@ -697,7 +704,8 @@ struct BatchWork {
   // key
   const Pc* P = nullptr;
   int pc_kind = -1, jac_k = 0;
-  int count = 0, small_rows = 0, refine = 0, cs = 0, g = 0;
+  int count = 0, refine = 0;
+  BatchShape shape;
   unsigned long long off_hash = 0;
   const double* x = nullptr;
   const double* b = nullptr;
@@ -732,6 +740,34 @@ void batch_work_free(Ctx* ctx, BatchWork* w) {
   delete w;
 }
 
+// The shape for systems of these sizes.  All systems together are to end at the
+// same time, so the largest one's threads are its share of the chip's: clusters
+// of 8 CTAs with 256, 512 or 1024 threads (2, 4 or 8 SMs' worth), and one CTA
+// for a system whose share is one CTA's threads or less.  Random graphs of mean
+// degree 20, diagonal PCG to 1e-8, FP64, B200, ms with 256 / 512 / 1024 threads
+// (in brackets the former fixed shape, 4 CTAs of 256 threads): 96 systems of
+// 1,000-65,536 rows 8.1 / 5.7 / 6.7 (16.3), 32 of them 7.1 / 5.0 / 4.4 (13.1), 16 of
+// 20,000 rows 3.3 / 2.4 / 2.1 (5.5), 300 of 8,000 6.1 / 7.0 / 9.4 (6.9), 1,024 of
+// 3,000 6.7 / 7.1 / 8.4 (7.5).  Solved by one CTA below 4,096 / 2,048 / 1,024 rows:
+// the 96 systems 6.2 / 5.7 / 5.5 (512 threads), the 1,024 systems 6.7 / 8.5 / 8.5 (256);
+// 100 systems of 1,500 rows 1.9 / 1.9 / 0.76 (their share is 1,516 threads).
+// The stream product takes the rows of a warp together: 3-10 % faster than 8
+// lanes per row here, but one lane adds up a row, so only for rows that fit its
+// chunk of 256 entries.
+BatchShape batched_shape(const Csr* A, int count, const int32_t* h_off) {
+  int most = 0;
+  for (int s = 0; s < count; ++s) most = std::max(most, h_off[s + 1] - h_off[s]);
+  const double n = std::max(A->n_rows, 1), chip = A->ctx->num_sms * 1024.0;
+  const double share = most / n * chip;
+  BatchShape shape;
+  shape.cs = 8;
+  shape.threads = share <= 2048 ? 256 : share <= 8192 ? 512 : 1024;
+  shape.g = A->max_row <= 32 * kStreamChunk ? 1 : 8;
+  shape.small_rows = (int)std::min(shape.threads == 256 ? 4096.0 : 2048.0,
+                                   std::ceil(shape.threads * n / chip));
+  return shape;
+}
+
 // Drops the cached batched configuration of A (all of it, or only if it
 // uses preconditioner only_P).
 void release_batch_work(Csr* A, const Pc* only_P) {
@@ -760,8 +796,9 @@ BatchVecs<T> carve(char* vecs, size_t vec_bytes) {
 }
 
 mtlgpu_status batch_work_build(Csr* A, Pc* P, int count, const int32_t* h_off, double* d_x,
-                               const double* d_b, const mtlgpu_iter_params* prm, int cs, int g,
-                               int small_rows, BatchWork* w) {
+                               const double* d_b, const mtlgpu_iter_params* prm, const BatchShape& shape,
+                               BatchWork* w) {
+  const int cs = shape.cs, g = shape.g, threads = shape.threads, small_rows = shape.small_rows;
   Ctx* ctx = A->ctx;
   const bool refine = w->refine;
   const int n = A->n_rows;
@@ -830,7 +867,8 @@ mtlgpu_status batch_work_build(Csr* A, Pc* P, int count, const int32_t* h_off, d
   a.inner_max = prm->inner_max_iter > 0 ? prm->inner_max_iter : prm->max_iter;
   a.max_outer = prm->max_outer > 0 ? prm->max_outer : 30;
   a.g = g;
-  int mc = refine ? clusters_for<float>(g, cs) : clusters_for<double>(g, cs);
+  int mc = refine ? clusters_for<float>(g, cs, threads)
+                  : clusters_for<double>(g, cs, threads);
   if (mc <= 0) return MTLGPU_NOT_SUPPORTED;
   // persistent: as many clusters as fit the GPU at once (phase 2 keeps every
   // CTA busy on small systems once the large ones are taken)
@@ -844,9 +882,9 @@ mtlgpu_status batch_work_build(Csr* A, Pc* P, int count, const int32_t* h_off, d
   if (e == cudaSuccess)
     e = cudaMemsetAsync(w->d_state, 0, sizeof(BatchState) * count, ctx->stream);
   if (e == cudaSuccess)
-    e = refine ? launch_g<float>(ctx->stream, g, cs, clusters, a,
+    e = refine ? launch_cluster<float>(ctx->stream, g, cs, threads, clusters, a,
                                  carve<float>(w->vecs, vec_bytes), 1)
-               : launch_g<double>(ctx->stream, g, cs, clusters, a,
+               : launch_cluster<double>(ctx->stream, g, cs, threads, clusters, a,
                                   carve<double>(w->vecs, vec_bytes), 0);
   mtlgpu_status st = MTLGPU_OK;
   if (e == cudaSuccess) {
@@ -881,7 +919,7 @@ mtlgpu_status batch_work_build(Csr* A, Pc* P, int count, const int32_t* h_off, d
 
 mtlgpu_status solve_batched_cluster(Csr* A, Pc* P, int count, const int32_t* h_off, double* d_x,
                                     const double* d_b, const mtlgpu_iter_params* prm,
-                                    mtlgpu_iter_result* res, int cs, int g, int small_rows,
+                                    mtlgpu_iter_result* res, const BatchShape& shape,
                                     float* ms_out) {
   Ctx* ctx = A->ctx;
   const bool refine = prm->mode == MTLGPU_SOLVE_MIXED_REFINED;
@@ -900,18 +938,18 @@ mtlgpu_status solve_batched_cluster(Csr* A, Pc* P, int count, const int32_t* h_o
            v->max_outer == prm->max_outer;
   };
   if (!w || w->P != P || w->pc_kind != pk || w->jac_k != jk || w->count != count ||
-      w->small_rows != small_rows || w->refine != (int)refine || w->cs != cs || w->g != g ||
+      !(w->shape == shape) || w->refine != (int)refine ||
       w->off_hash != hsh || w->x != d_x || w->b != d_b || w->val32 != A->d_v32 || !same_params(w)) {
     release_batch_work(A, nullptr);
     w = new BatchWork();
-    w->P = P, w->pc_kind = pk, w->jac_k = jk, w->count = count, w->small_rows = small_rows;
-    w->refine = refine, w->cs = cs, w->g = g, w->off_hash = hsh, w->x = d_x, w->b = d_b;
+    w->P = P, w->pc_kind = pk, w->jac_k = jk, w->count = count, w->shape = shape;
+    w->refine = refine, w->off_hash = hsh, w->x = d_x, w->b = d_b;
     w->val32 = A->d_v32;
     w->rtol = prm->rtol, w->atol = prm->atol, w->inner_rtol = prm->inner_rtol;
     w->max_iter = prm->max_iter, w->inner_max = prm->inner_max_iter;
     w->max_outer = prm->max_outer;
     A->batch_work = w;
-    mtlgpu_status st = batch_work_build(A, P, count, h_off, d_x, d_b, prm, cs, g, small_rows, w);
+    mtlgpu_status st = batch_work_build(A, P, count, h_off, d_x, d_b, prm, shape, w);
     if (st != MTLGPU_OK) {
       release_batch_work(A, nullptr);
       return st;

@@ -98,6 +98,16 @@ struct WorkspaceEntry {
   void* ws;
 };
 
+// How a batched solve is split (batched_cluster.cu): CTAs per large system (the
+// cluster size; 0: chosen from the systems), lanes per matrix row (1: the stream
+// product), threads per CTA, and the rows below which one CTA solves a system.
+struct BatchShape {
+  int cs = 0, g = 0, threads = 256, small_rows = 0;
+  bool operator==(const BatchShape& o) const {
+    return cs == o.cs && g == o.g && threads == o.threads && small_rows == o.small_rows;
+  }
+};
+
 struct Csr {
   Ctx* ctx = nullptr;
   std::vector<WorkspaceEntry> workspaces;
@@ -122,10 +132,7 @@ struct Csr {
   int n_blk = 0;
   int spmv_kernel = 0;             // 0 = CSR-stream, 1 = row-binned groups, 2 = SELL-32
   Sell sell;                       // SELL-32 copy (spmv_kernel == 2)
-  // batched solves: CTAs per system (cluster size), lanes per row, and the
-  // row count below which a system is solved by one CTA; picked by
-  // mtlgpu_batched_autotune
-  int batch_cs = 4, batch_g = 8, batch_small = 4096;
+  BatchShape batch;                // of batched solves, from mtlgpu_batched_autotune
   void* batch_work = nullptr;      // cached batched configuration (batched_cluster.cu)
   // transpose (built on demand for A^T x)
   int32_t* d_trp = nullptr;
@@ -261,9 +268,10 @@ mtlgpu_status csr_autotune_spmv(Csr* A, int* choice, float* ms);
 // Batched PCG in one persistent cluster launch (batched_cluster.cu).
 bool batched_cluster_supported(const Pc* P);
 void release_batch_work(Csr* A, const Pc* only_P);
+BatchShape batched_shape(const Csr* A, int count, const int32_t* h_off);
 mtlgpu_status solve_batched_cluster(Csr* A, Pc* P, int count, const int32_t* h_off, double* d_x,
                                     const double* d_b, const mtlgpu_iter_params* prm,
-                                    mtlgpu_iter_result* res, int cs, int g, int small_rows,
+                                    mtlgpu_iter_result* res, const BatchShape& shape,
                                     float* ms_out);
 
 // Sweeps (sweep.cu): out must be prefilled with the sentinel when
