@@ -14,7 +14,9 @@
 //        r', whose gathers form r'[c] = r[c] - alpha q[c] on the fly;
 //   K_B  the remaining passes, the U triangle and rho = r'.z (unchanged);
 //   K_C  p' = z + beta p formed on the fly at every gathered column, written
-//        for the own row, q = A p' and p'.q (last block: alpha_1).
+//        for the own row, q = A p' and p'.q (last block: alpha_1); from 2^20 rows
+//        of a stencil matrix on, a pass for p' and the plain product instead
+//        (direction_split).
 // r and p are double-buffered (the kernels that write r' and p' gather the
 // old vectors), x is updated in place (row-local).  Every value of r' and
 // p' is produced by one helper, so a gathered value and the stored one are
@@ -321,6 +323,28 @@ __global__ void __launch_bounds__(kBlock, kGridBlocksC)
   }
 }
 
+// p' = z + beta p on its own (direction_split).  Bound by HBM: three vectors.
+template <typename T>
+__global__ void __launch_bounds__(kBlock, 8)
+    cg_direction_kernel(int n, const T* __restrict__ z, const T* __restrict__ p,
+                        T* __restrict__ p_next, const SolverState* st) {
+  if (st->done) return;
+  constexpr int V = VN<T>::value;
+  const T beta = (T)(st->rho / st->rho_1);
+  for (long long i0 = gtid() * V; i0 < n; i0 += gstride() * V) {
+    if (i0 + V <= n) {
+      T zv[V], pv[V];
+      ld16(z + i0, zv);
+      ld16(p + i0, pv);
+#pragma unroll
+      for (int u = 0; u < V; u++) pv[u] = next_p(zv[u], pv[u], beta);
+      st16(p_next + i0, pv);
+    } else {
+      for (long long i = i0; i < n; i++) p_next[i] = next_p(z[i], p[i], beta);
+    }
+  }
+}
+
 template <typename T>
 struct Vals;
 template <>
@@ -431,6 +455,15 @@ __global__ void __launch_bounds__(kBlock, grid_blocks_t<T>())
     }
   }
 }
+
+// Whether p' is made by a pass of its own and the product gathers p' alone.  K_C
+// gathers two vectors per entry: on the grid layout, whose product is otherwise
+// bound by memory, that costs more than p' written and read again once the
+// launch it saves (~2 us) weighs less.  One iteration, K_C / split, us (FP64; FP32
+// of the mixed solve): 7-point 64^3 24.8 / 25.6; 23.4 / 25.7, 96^3 46.9 / 45.6;
+// 38.4 / 38.0, 128^3 96.0 / 91.6; 68.3 / 66.0, 144^3 135.8 / 126.1; 91.7 / 86.5; 5-point
+// 1024^2 44.0 / 44.4; 37.0 / 36.5, 1400^2 77.4 / 76.2; 57.8 / 54.9.
+bool direction_split(const Sell& S) { return S.grid && S.n >= 1 << 20; }
 
 struct BetaSrc {
   const int* skip;
@@ -570,6 +603,17 @@ mtlgpu_status cg_fused_iteration(Csr* A, Pc* P, SolverState* st, T* x, const T* 
   Ctx* ctx = A->ctx;
   MTLGPU_TRY((fused_apply<T, false>(ctx, P, st, x, p, r, q, r_next, z, &st->done, r_next,
                                     &st->rho)));
+  if (direction_split(A->sell)) {
+    const int grid = rows_grid(ctx, (A->n_rows + VN<T>::value - 1) / VN<T>::value, 8);
+    cg_direction_kernel<T><<<grid, kBlock, 0, ctx->stream>>>(A->n_rows, z, p, p_next, st);
+    ctx->launches++;
+    SpmvArgs a;
+    a.epi = EPI_DOT_X2;
+    a.x2 = p_next;
+    a.out = &st->alpha_1;
+    a.skip = &st->done;
+    return spmv_launch<T>(A, p_next, q, a);
+  }
   launch_pspmv<T, false>(ctx, A->sell, Vals<T>::val(A->sell), z, p, p_next, q, state_beta(st));
   MTLGPU_TRY_CUDA(ctx, cudaGetLastError());
   return MTLGPU_OK;
