@@ -130,6 +130,21 @@ def sell_index_bytes(rp, ci):
     return 2 if int(np.abs(ci.astype(np.int64) - rows).max()) <= 32767 else 4
 
 
+def layout_bytes(rp, ci):
+    """(bytes of index per entry, bytes per row) of the layout the products and
+    Jacobi applies read, beside the values and vectors: the grid layout (a mask
+    of 1, 2 or 4 bytes per row, nothing per entry) where the matrix has at most
+    32 offsets and padding every row to all of them adds at most a quarter;
+    else SELL-32 (sell_index_bytes and a 4-byte offset per 32 rows)."""
+    n = len(rp) - 1
+    if os.environ.get("MTLGPU_SELL_INDEX", "") != "32" and len(ci):
+        rows = np.repeat(np.arange(n, dtype=np.int64), np.diff(rp))
+        w = len(np.unique(ci - rows))
+        if w <= 32 and w * n <= 1.25 * len(ci):
+            return 0, 1 if w <= 8 else 2 if w <= 16 else 4
+    return sell_index_bytes(rp, ci), 4 / 32
+
+
 def problem(M):
     A = M.laplacian3d(N_GRID)
     xt = M.uniform(A[0], 1)
@@ -917,37 +932,38 @@ def main():
         torch.cuda.synchronize()
         return sum(a.elapsed_time(b) for a, b in evs) / reps_
 
-    def spmv_stats(dA_, n_, nnz_, ib_, reps_=100):
-        # algorithmic bytes: 8-byte value + ib_-byte index per entry, the
-        # slice offsets, x once and y once
+    def spmv_stats(dA_, n_, nnz_, layout, reps_=100):
+        # algorithmic bytes: 8-byte value and the layout's index bytes per
+        # entry, its bytes per row, x once and y once
+        ib_, rb_ = layout
         dxs, dys = ctx.to_device(M.uniform(n_, 5)), ctx.array(n_)
         for _ in range(5):
             dA_.spmv(dxs, dys)
         ms, _ = timed(lambda: dA_.spmv(dxs, dys), reps_)
         ms_cold = cold_ms(lambda: dA_.spmv(dxs, dys), 30)
-        byt = nnz_ * (8 + ib_) + 4 * (n_ // 32 + 1) + 2 * n_ * 8
+        byt = int(nnz_ * (8 + ib_) + rb_ * n_) + 2 * n_ * 8
         return {"ms": ms, "GBps": byt / ms / 1e6, "hbm_frac": byt / ms / 1e6 / peak,
-                "bytes": byt, "index_bytes": ib_, "peak_kind": peak_kind,
+                "bytes": byt, "index_bytes": ib_, "row_bytes": rb_, "peak_kind": peak_kind,
                 "back_to_back": "mean of %d products back to back" % reps_,
                 "cold": {"ms": ms_cold, "GBps": byt / ms_cold / 1e6,
                          "hbm_frac": byt / ms_cold / 1e6 / peak,
                          "how": "L2 flushed before each product, per-launch CUDA events"}}
 
-    ib = sell_index_bytes(A[1], A[2])
-    spmv = spmv_stats(dA, n, nnz, ib)
+    ib, rb = layout = layout_bytes(A[1], A[2])
+    spmv = spmv_stats(dA, n, nnz, layout)
 
     # The mixed solve's kernels, timed alone on the same data (FP32).  Per
-    # inner iteration the solve runs three: the direction product
-    # (p = z + beta p, q = A p, p.q), the first L pass fused with the x / r
-    # update, and the U pass with r.z; the first and the last are timed here
-    # (the fused L pass has no entry point of its own; its share is in the
-    # launch-list profile).  Algorithmic bytes: the product reads A's entries
-    # (4-byte value + ib-byte index), the slice offsets, z and p once and
-    # writes p and q; a Jacobi pass reads the factor's off-diagonal entries
-    # (4-byte value + ib-byte index), v, D and the previous iterate once and
-    # writes one vector.  The plain FP32 SpMV is timed for the record.
+    # inner iteration the solve runs the product with p.q after a pass for
+    # p = z + beta p (stencil matrices of 2^20 rows and more; below, both in one
+    # kernel, mtlgpu_cg_direction_product), the first L pass fused with the x / r
+    # update, and the U pass with r.z; the product and the U pass are timed
+    # here (the fused L pass has no entry point of its own).  Algorithmic
+    # bytes: the product reads A's 4-byte values, the layout's index bytes and x
+    # and writes y; a Jacobi pass reads the factor's off-diagonal entries, v, D
+    # and the previous iterate once and writes one vector.
     nnz_off = P32.factor_info(M.LOWER)[0] - n
-    bytes_pass = nnz_off * (4 + ib) + 4 * (n // 32 + 1) + 4 * n * 4
+    rb_tri = min(rb, 2) if ib == 0 else rb
+    bytes_pass = int(nnz_off * (4 + ib) + rb_tri * n) + 4 * n * 4
     r32 = ctx.to_device(np.ones(n, np.float32))
     z32 = ctx.array(n, np.float32)
     for _ in range(3):
@@ -959,8 +975,11 @@ def main():
     y32 = ctx.array(n, np.float32)
     for _ in range(5):
         dA.spmv_f32(x32, y32)
-    ms_spmv32, _ = timed(lambda: dA.spmv_f32(x32, y32), 100)
-    bytes_spmv32 = nnz * 8 + 4 * (n // 32 + 1) + 2 * n * 4   # 4-byte indices in FP32
+    ms_spmv32_b2b, _ = timed(lambda: dA.spmv_f32(x32, y32), 100)
+    ms_spmv32 = after_ms(lambda: dA.spmv_f32(x32, y32), lambda: P32.apply_f32(r32, z32), 50)
+    ms_spmv32_cold = cold_ms(lambda: dA.spmv_f32(x32, y32), 30)
+    # SELL-32: 4-byte indices in FP32
+    bytes_spmv32 = int(nnz * (4 if ib == 0 else 8) + rb * n) + 2 * n * 4
     p32, po32, q32, dpq = (ctx.to_device(M.uniform(n, 6).astype(np.float32)),
                            ctx.array(n, np.float32), ctx.array(n, np.float32), ctx.array(1))
 
@@ -969,13 +988,14 @@ def main():
 
     for _ in range(5):
         direction()
-    # In the solve the product follows the IC(0) apply (L and U passes,
-    # ~150 MB streamed): timed that way for the roofline; back to back (L2
-    # keeps part of A between launches) and with L2 flushed, for the record.
+    # In the solve the products follow the IC(0) apply (L and U passes): timed
+    # that way for the roofline; back to back (L2 keeps part of A between
+    # launches) and with L2 flushed, for the record.
     ms_dir32 = after_ms(direction, lambda: P32.apply_f32(r32, z32), 50)
     ms_dir32_b2b, _ = timed(direction, 100)
     ms_dir32_cold = cold_ms(direction, 30)
-    bytes_dir32 = nnz * (4 + ib) + 4 * (n // 32 + 1) + 4 * n * 4
+    bytes_dir32 = int(nnz * (4 + ib) + rb * n) + 4 * n * 4
+    split = ib == 0 and n >= 1 << 20
     traffic = read_traffic()
 
     # exact sweeps (the FP64 path's dominant kernel), for the record
@@ -1002,11 +1022,12 @@ def main():
     ms_e2e = max_over_ranks(ms_e2e)
 
     dominant = {
-        "jacobi_pass_kernel<float> (IC(0) U pass, r.z fused)": (ms_pass, bytes_pass,
-                                                                 2 * JACOBI_K - 1,
-                                                                 "jacobi_pass_f32"),
-        "cg_pspmv_kernel<float> (p = z + beta p, q = A p, p.q)": (ms_dir32, bytes_dir32, 1,
-                                                                   "cg_pspmv_f32"),
+        "Jacobi pass, FP32 (IC(0) U pass, r.z fused)": (ms_pass, bytes_pass, 2 * JACOBI_K - 1,
+                                                         "jacobi_pass_f32"),
+        "product, FP32 (q = A p)": (ms_spmv32, bytes_spmv32, int(split), "spmv_f32"),
+        "direction product, FP32 (p = z + beta p, q = A p, p.q)": (ms_dir32, bytes_dir32,
+                                                                    int(not split),
+                                                                    "cg_pspmv_f32"),
     }
     dom = max(dominant, key=lambda k: dominant[k][0] * dominant[k][2])
     d_ms, d_bytes, _, d_key = dominant[dom]
@@ -1024,7 +1045,8 @@ def main():
         "dtype": "f32+f64",
         "data": "synthetic",
         "config": {"workload": WORKLOAD, "n": n, "nnz": nnz,
-                   "index": "int32 CSR; SELL-32 column indices: %d bytes in the solve's "
+                   "index": "int32 CSR; grid layout, %d-byte mask per row" % rb if ib == 0 else
+                            "int32 CSR; SELL-32 column indices: %d bytes in the solve's "
                             "kernels and the FP64 SpMV, 4 in the plain FP32 SpMV" % ib,
                    "jacobi_iterations_per_triangle": JACOBI_K, "inner_rtol": INNER_RTOL,
                    "l2": "inputs larger than L2 (matrix 175 MB + factors 2 x 100 MB)",
@@ -1047,7 +1069,7 @@ def main():
         "mixed_kernels": {"cg_pspmv_f32": {"ms": ms_dir32, "GBps": bytes_dir32 / ms_dir32 / 1e6,
                                            "how": "each launch right after an IC(0) apply, "
                                                   "as in the solve; per-launch CUDA events",
-                                           "bytes": bytes_dir32, "launches_per_iteration": 1,
+                                           "bytes": bytes_dir32, "launches_per_iteration": int(not split),
                                            "back_to_back_ms": ms_dir32_b2b,
                                            "cold_ms": ms_dir32_cold,
                                            "cold_GBps": bytes_dir32 / ms_dir32_cold / 1e6},
@@ -1057,7 +1079,10 @@ def main():
                                               "cold_ms": ms_pass_cold,
                                               "cold_GBps": bytes_pass / ms_pass_cold / 1e6},
                           "spmv_f32": {"ms": ms_spmv32, "GBps": bytes_spmv32 / ms_spmv32 / 1e6,
-                                       "bytes": bytes_spmv32}},
+                                       "how": "each launch right after an IC(0) apply",
+                                       "bytes": bytes_spmv32, "launches_per_iteration": int(split),
+                                       "back_to_back_ms": ms_spmv32_b2b,
+                                       "cold_ms": ms_spmv32_cold}},
         "sweep_fp64": {"ms": ms_sweep64, "GBps": bytes_sweep64 / ms_sweep64 / 1e6,
                        "bytes": bytes_sweep64, "levels": P64.factor_info(M.LOWER)[1]},
         "setup_s": {"total": setup_s, "ic0_fp64": t_fac64, "ic0_fp32": t_fac32},
@@ -1132,7 +1157,7 @@ def config3_workload(M, ctx, timed, solver, spmv_stats, peak):
                           "mixed_outer": rmx[-1].outer_iterations},
            "true_rel_residual": float(np.linalg.norm(b - M.csr_mult(A, x)) / np.linalg.norm(b)),
            "jacobi_iterations_per_triangle": JACOBI_K,
-           "spmv": spmv_stats(dA, n, nnz, sell_index_bytes(A[1], A[2]))}
+           "spmv": spmv_stats(dA, n, nnz, layout_bytes(A[1], A[2]))}
     P32.close()
     P64.close()
     dA.close()

@@ -246,7 +246,7 @@ mtlgpu_status mtlgpu_csr_values_grad(mtlgpu_csr* A, const double* d_lambda, cons
 /* Choose the SpMV layout of this matrix by timing the bit-exact candidates
  * on it (CUDA events, 20 products each): SELL-32 where its padding is at most
  * 2 nnz, and the CSR-stream row blocks.  The fastest is kept on the handle;
- * *h_choice (when non-NULL) receives 2 (SELL-32) or 0 (CSR-stream).  No
+ * *h_choice (when non-NULL) receives 2 (SELL-32 or grid) or 0 (CSR-stream).  No
  * counterpart in the reference (the layout behind mat_vec_mult.hpp:620-689). */
 mtlgpu_status mtlgpu_csr_autotune(mtlgpu_csr* A, int* h_choice);
 
