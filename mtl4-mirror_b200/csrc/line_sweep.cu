@@ -43,15 +43,16 @@
 // issue of the warp's ~32 instructions.  So a step's operands are read a step
 // ahead, a block's inputs are asked for during the block before, a block whose
 // lanes all have rows has no tests per row, and records lie in memory as the
-// stages have them, one bulk copy per stage: 88 instructions and 240 cycles a
+// stages have them, one bulk copy per stage: 51 instructions and 240 cycles a
 // step before that (FP64, 512^2; 377 cycles at 128^3).  A tile boundary costs
 // 1.5-2.5 us: a store to L2, a poll, the inbox, and the rest of a block on both
 // sides.  One call of the lower sweep (~25 us of it the fill and the host's wait),
 // level-ordered / before / now: 128^3 7-point 546 / 175 / 152 us (FP32 517 / 135 /
 // 123), 96^3 27-point 850 / 365 / 279, 512^2 5-point 1,145 / 147 / 109, 100^2
 // 224 / 52 / 47.  Slower: blocks of 2 steps (512^2 144, 128^3 152-181), of 8 (128^3
-// 190 with the former kernel), and a chunk counter by cp.async groups in place of
-// the stages' mbarriers (the loader then waits for each copy).  Earlier forms on
+// 190 with the former kernel), a counter by cp.async groups in place of the
+// stages' mbarriers (the loader then waits for each copy), and results stored two
+// rows at a time (512^2 177, 128^3 184).  Earlier forms on
 // 512^2: lanes advancing independently 830 us; lanes in step with tagged slots
 // polled and voted on per row 281.
 //

@@ -60,7 +60,9 @@ CASES = [((8, 8), False), ((9, 31), False), ((32, 33), False), ((65, 8), False),
          ((4, 8, 8), False), ((5, 9, 11), False), ((17, 16, 13), False), ((2, 3, 40), False),
          ((33, 8, 10), False), ((20, 35, 9), False),
          ((4, 8, 8), True), ((5, 9, 11), True), ((17, 16, 13), True), ((2, 3, 40), True),
-         ((33, 9, 8), True), ((18, 33, 10), True)]
+         ((33, 9, 8), True), ((18, 33, 10), True),
+         # more tiles of 8 x 8 lines than SMs: the 16 x 8 form
+         ((97, 105, 8), False), ((75, 101, 9), True)]
 
 
 @pytest.mark.parametrize("dims,box", CASES)
