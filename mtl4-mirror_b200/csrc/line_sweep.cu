@@ -90,6 +90,7 @@
 
 #include "device.cuh"
 #include "internal.h"
+#include "line_tiles.h"
 #include "tma.cuh"
 
 namespace mtlgpu {
@@ -251,7 +252,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     s_done = 0;
   }
   __syncthreads();
-  const int I0 = s_tile / A.ntj * A.TI, J0 = s_tile % A.ntj * A.TJ;
+  const int trow = s_tile / A.ntj, I0 = trow * A.TI;
+  const int J0 = (line_tile_col0(trow, A.TI, A.TJ, S::sk) + s_tile % A.ntj) * A.TJ;
   // first row (in x order) of the line at (gi, gj) of the tile, -1 outside the grid
   auto line_first = [&](int gi, int gj) {
     const int i = I0 + gi, j = J0 + gj - i * S::sk;
@@ -553,7 +555,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     // the block of the patch's first row
     const int b0 = skew_of(cw / npj * S::PI, cw % npj * S::PJ) / KL;
     const unsigned char* rec0 =
-        recs + ((long long)(s_tile * A.compute_warps + cw) * A.blocks - b0) * kStage;
+        recs + (((long long)s_tile * A.compute_warps + cw) * A.blocks - b0) * kStage;
     long long polls = 0;
     bool stop = false;
     int blk = 0;
@@ -662,7 +664,8 @@ __global__ void line_fill_kernel(const __grid_constant__ LineShape L,
     const int js = j + i * S::sk, gi = i % A.TI, gj = js % A.TJ;
     const int pi = gi / S::PI, pj = gj / S::PJ, npj = A.TJ / S::PJ;
     const int step = t + S::skew(gi, gj), b0 = S::skew(pi * S::PI, pj * S::PJ) / KL;
-    const long long warp = (long long)(i / A.TI * A.ntj + js / A.TJ) * A.compute_warps + pi * npj + pj;
+    const long long warp =
+        line_tile_of(i, js, A.TI, A.TJ, S::sk, A.ntj) * A.compute_warps + pi * npj + pj;
     const int lane = gi % S::PI * S::PJ + gj % S::PJ;
     unsigned char* o = rec + (((warp * A.blocks + step / KL - b0) * KL + step % KL) * kPpr * 32 + lane) * 16;
     int q = rp[r];
@@ -755,9 +758,9 @@ bool line_layout_t(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
   // patch.  Stages: four where they fit, else two (16 x 8 lines in FP64: the same
   // time).
   A->TJ = S::PJ;
-  A->ntj = (L.P + (L.NI - 1) * S::sk + A->TJ - 1) / A->TJ;
   A->TI = !S::amax ? 1 : G == 4 && ts == 8 ? 4 : 8;
-  if (A->TI == 8 && (L.NI + 7) / 8 * A->ntj > ctx->num_sms) A->TI = 16;
+  auto tiles = [&] { return line_tile_count(L.P, L.NI, A->TI, A->TJ, S::sk); };
+  if (A->TI == 8 && tiles() > ctx->num_sms) A->TI = 16;
   const int limit = smem_limit(ctx);
   for (A->stages = 4;; A->stages == 4 ? A->stages = 2 : (A->stages = 4, A->TI /= 2)) {
     if (A->TI < S::PI) return false;
@@ -782,7 +785,9 @@ bool line_layout_t(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
     A->smem = o;
     if (o <= limit && (2 * A->compute_warps + A->fetch_warps) * 32 <= kMaxThreads) break;
   }
-  A->ntiles = A->ntj * ((L.NI + A->TI - 1) / A->TI);
+  if (tiles() > INT32_MAX) return false;
+  A->ntj = line_tile_cols(L.P, L.NI, A->TI, A->TJ, S::sk);
+  A->ntiles = (int)tiles();
   // the last line's last step makes the zero row past its end
   const int skew = (A->TJ - 1) * S::s1 + (A->TI - 1) * S::s2 +
                    (A->TJ / S::PJ + A->TI / S::PI - 2) * S::X + 1;
