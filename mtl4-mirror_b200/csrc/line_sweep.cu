@@ -796,10 +796,15 @@ bool line_layout_t(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
   A->blocks = (S::kLoad - 1 + S::skew(S::PI - 1, S::PJ - 1) - S::skew(0, 0) + L.B - 1) / S::kLoad + 1;
   return true;
 }
-bool line_layout(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
-  if (L.E == 1)
-    return L.G == 1 ? line_layout_t<1, 1>(ctx, L, ts, A) : line_layout_t<2, 1>(ctx, L, ts, A);
-  return L.G == 1 ? line_layout_t<1, 3>(ctx, L, ts, A) : line_layout_t<4, 3>(ctx, L, ts, A);
+size_t record_bytes(const LineArgs& A) {
+  return (size_t)A.ntiles * A.compute_warps * A.blocks * A.stage;
+}
+bool line_layout(Ctx* ctx, const LineShape& L, int ts, size_t device, LineArgs* A) {
+  const bool fits =
+      L.E == 1 ? (L.G == 1 ? line_layout_t<1, 1>(ctx, L, ts, A) : line_layout_t<2, 1>(ctx, L, ts, A))
+               : (L.G == 1 ? line_layout_t<1, 3>(ctx, L, ts, A) : line_layout_t<4, 3>(ctx, L, ts, A));
+  return fits && line_records_fit((long long)L.n * A->rec_bytes, (long long)record_bytes(*A),
+                                  (long long)device);
 }
 
 template <typename T>
@@ -933,7 +938,10 @@ mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* P, const SweepPlan* like, co
   dfree(ctx, d_s);
   MTLGPU_TRY(st);
   LineArgs A[2];
-  if (!found || !line_layout(ctx, S, 8, &A[0]) || !line_layout(ctx, S, 4, &A[1])) return MTLGPU_OK;
+  size_t free_bytes = 0, device = 0;
+  MTLGPU_TRY_CUDA(ctx, cudaMemGetInfo(&free_bytes, &device));
+  if (!found || !line_layout(ctx, S, 8, device, &A[0]) || !line_layout(ctx, S, 4, device, &A[1]))
+    return MTLGPU_OK;
   LinePlan* L = new LinePlan();
   P->line = L;
   L->shape = S;
@@ -962,7 +970,7 @@ mtlgpu_status line_plan_fill(Ctx* ctx, SweepPlan* P, int prec, const int32_t* d_
   const LineArgs& A = L.args[prec];
   unsigned char* rec = static_cast<unsigned char*>(L.d_rec[prec]);
   if (!rec) {
-    MTLGPU_TRY(dalloc(ctx, &rec, (size_t)A.ntiles * A.compute_warps * A.blocks * A.stage));
+    MTLGPU_TRY(dalloc(ctx, &rec, record_bytes(A)));
     L.d_rec[prec] = rec;
   }
   if (prec)

@@ -43,4 +43,15 @@ MTLGPU_HD long long line_tile_of(int i, int js, int TI, int TJ, int sk, int cols
   return (long long)ti * cols + js / TJ - line_tile_col0(ti, TI, TJ, sk);
 }
 
+// Whether a factor's records may take `padded` bytes where its rows' own take
+// `own`.  Lanes without a line and stages without a row are stored too: a plane of
+// two lines takes 16 times its rows, lines of 8 rows 4 to 6 times.  Grids of ordinary
+// shape stay below twice their rows.  Thin ones keep their records while these are a
+// small part of the device's memory (a level-ordered sweep of such a grid has as
+// many levels as the grid is long, and takes 1.3 us for each); beyond that their
+// sweeps go by levels, at a few dozen bytes per row.
+inline bool line_records_fit(long long own, long long padded, long long device) {
+  return padded <= 4 * own || padded <= device / 32;
+}
+
 }  // namespace mtlgpu

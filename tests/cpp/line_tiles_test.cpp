@@ -56,5 +56,15 @@ int main() {
   grid(3, 370728, 4, 8, 1, false);
   grid(3, 80000000, 4, 8, 1, false);
   check(line_tile_count(3, 370728, 4, 8, 1) <= 2ll * 370728 / 4, "linear", 3, 370728, 4, 8, 1);
+  // records: up to four times the rows' own, or a 32nd of the device
+  const long long device = 180ll << 30, part = device / 32;
+  for (long long own : {1ll << 20, part / 4 + 1, 40ll << 30})
+    for (long long f : {1, 4, 5, 16}) {
+      const bool fits = line_records_fit(own, f * own, device);
+      if (fits != (f <= 4 || f * own <= part)) {
+        std::printf("records %lld x %lld\n", own, f);
+        return 1;
+      }
+    }
   std::puts("ok");
 }
