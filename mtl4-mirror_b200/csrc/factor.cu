@@ -589,7 +589,10 @@ mtlgpu_status build_ilu0(Pc* P) {
 
 // The exact sweeps of P in precision `prec` ready to launch: for grid-line
 // plans the records, made at the first exact solve (factors applied by Jacobi
-// iterations alone never need them).  Call before any stream capture.
+// iterations alone never need them).  FP32 records are made with the
+// preconditioner: mtlgpu_pc_apply_f32 does not wait for the stream, so its first
+// call may be inside a capture, where nothing can be allocated.  Call before any
+// stream capture.
 mtlgpu_status pc_ensure_sweeps(Pc* P, int prec) {
   if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0)) return MTLGPU_OK;
   Ctx* ctx = P->A->ctx;
@@ -648,6 +651,7 @@ mtlgpu_status pc_build(Pc* P) {
   const bool f32 = P->prec == MTLGPU_FP32;
   MTLGPU_TRY(part_plan_build(ctx, &P->lower, f32));
   MTLGPU_TRY(part_plan_build(ctx, &P->upper, f32));
+  if (f32) MTLGPU_TRY(pc_ensure_sweeps(P, MTLGPU_FP32));
   return take_device_error(ctx);
 }
 
