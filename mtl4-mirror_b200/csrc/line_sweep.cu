@@ -80,8 +80,8 @@
 // Progress: tiles are claimed by an atomic ticket in an order in which every
 // dependency points to the same or an earlier tile (lines shifted by `sk` per
 // plane where a stencil reaches forward in the previous plane), so a CTA only
-// waits for CTAs that run or have ended.  Every wait is bounded
-// (MTLGPU_TIMEOUT).
+// waits for CTAs that run or have ended.  Every wait is bounded by itself, from
+// the last row that came (MTLGPU_TIMEOUT): a long sweep is no long wait.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -500,6 +500,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     if (lane < A.compute_warps && !(fed >> lane & 1))
       st_shared_release(halo + (lane * A.fetch_warps + fw) * 4, kNever);
     int t = 0;
+    bool begun = false;
+    // polls: those since the last row filed
     for (long long polls = 0; polls < limit; ++polls) {
       const int row = t + sub;
       T v = ld_relaxed(o + (long long)dir * min(row, last));
@@ -519,7 +521,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       t += cnt;
       // the steps whose values from this warp's lines are all filed, per warp
       // (at first: those before the lines' row 0)
-      if (polls == 0 || __any_sync(0xffffffffu, cnt > 0)) {
+      const bool filed = __any_sync(0xffffffffu, cnt > 0);
+      if (filed) polls = -1;
+      if (!begun || filed) {
+        begun = true;
         __syncwarp();
         for (unsigned m = fed; m; m &= m - 1) {
           const int c = __ffs(m) - 1;
@@ -556,11 +561,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const int b0 = skew_of(cw / npj * S::PI, cw % npj * S::PJ) / KL;
     const unsigned char* rec0 =
         recs + (((long long)s_tile * A.compute_warps + cw) * A.blocks - b0) * kStage;
-    long long polls = 0;
     bool stop = false;
     int blk = 0;
     for (; blk < A.steps / KL; blk++) {
       const int st = blk & smask, s0 = blk * KL;
+      long long polls = 0;
       while (s0 + KL - ld_shared_acquire(prog + cw * 4) > A.stages * KL) {
         if (++polls >= limit || *(volatile int*)&s_done == A.compute_warps) {
           stop = true;

@@ -1,0 +1,32 @@
+"""The spin limit bounds one wait of a sweep along grid lines, not the polls of
+the whole sweep: lines of 100,000 rows (two tiles, so that one waits for the
+other) are swept with a limit that every single wait keeps far below and the
+sweep's polls together exceed many times over.  A step of the sweep takes ~60 ns,
+so it runs for 6 ms; a loader polls every ~70 ns (90,000 polls) and the second
+tile's fetch every ~0.5 us (12,000); the limit of 4,096 polls is 150 us or more."""
+import numpy as np
+import pytest
+
+from test_gpu_line_sweep import context
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+def test_limit_is_of_one_wait(M, dt):
+    c = context(M)
+    try:
+        A = M.Csr.laplacian2d(c, 40, 100000)
+        P = M.Pc(A, "ic0", M.FP32)
+        x, y = c.to_device(np.ones(A.n, dt)), c.array(A.n, dt)
+        want = {}
+        for which in (M.LOWER, M.UPPER):
+            P.sweep(which, x, y)
+            want[which] = y.download()
+        c.set_spin_limit(4096)
+        for which in (M.LOWER, M.UPPER):
+            P.sweep(which, x, y)
+            assert np.array_equal(y.download(), want[which])
+        P.close(), A.close()
+    finally:
+        c.close()
