@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       unsigned tb[G];
 #pragma unroll
       for (int g = 0; g < G; g++)  // one place: no wrap inside the block
-        tb[g] = E == 1 ? tgt[g] + ((tpos[g] + s0 * kSlot) & (R * kSlot - 1)) : tgt[g];
+        tb[g] = E == 1 ? tgt[g] + ((tpos[g] + (unsigned)s0 * kSlot) & (R * kSlot - 1)) : tgt[g];
 #pragma unroll
       for (int u = 0; u < KS; u++) {
         bool next = false;
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         for (int g = 0; g < G; g++) {
           if (tgt[g])
             sts(E == 1 ? tb[g] + u * kSlot
-                       : tb[g] + ((tpos[g] + (s0 + u) * kSlot) & (R * kSlot - 1)), hist[0]);
+                       : tb[g] + ((tpos[g] + (unsigned)(s0 + u) * kSlot) & (R * kSlot - 1)), hist[0]);
 #pragma unroll
           for (int x = E - 1; x > 0; x--) w[g][x] = w[g][x - 1];
           w[g][0] = nw[g];
