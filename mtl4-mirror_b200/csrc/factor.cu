@@ -655,19 +655,6 @@ mtlgpu_status pc_build(Pc* P) {
   return take_device_error(ctx);
 }
 
-// The adjoint factor's grid-line form, records included (its CSR arrays are
-// temporary).
-static mtlgpu_status adjoint_line_plan(Pc* P, SweepPlan* S, const int32_t* rp, const int32_t* ci,
-                                       const double* v) {
-  Ctx* ctx = P->A->ctx;
-  const bool f32 = P->prec == MTLGPU_FP32;
-  MTLGPU_TRY(line_plan_detect(ctx, S, S == &P->adj_upper ? &P->adj_lower : nullptr, rp, ci));
-  if (!S->line) return MTLGPU_OK;
-  MTLGPU_TRY(line_plan_fill(ctx, S, 0, rp, ci, v, f32));
-  if (f32) MTLGPU_TRY(line_plan_fill(ctx, S, 1, rp, ci, v, true));
-  return MTLGPU_OK;
-}
-
 mtlgpu_status pc_ensure_adjoint(Pc* P) {
   if (P->adj_built || P->kind != MTLGPU_PC_ILU0) return MTLGPU_OK;
   Ctx* ctx = P->A->ctx;
@@ -679,8 +666,15 @@ mtlgpu_status pc_ensure_adjoint(Pc* P) {
   MTLGPU_TRY(dalloc(ctx, &tci, P->nnz_U));
   MTLGPU_TRY(dalloc(ctx, &tv, P->nnz_U));
   MTLGPU_TRY(csr_transpose(ctx, n, n, P->nnz_U, P->d_Urp, P->d_Uci, P->d_Uv, trp, tci, tv));
-  MTLGPU_TRY(build_sweep_plan(ctx, n, trp, tci, tv, true, false, true, &P->adj_lower));
-  MTLGPU_TRY(adjoint_line_plan(P, &P->adj_lower, trp, tci, tv));
+  // U^T of a grid stencil has L's pattern: along grid lines, records at once (the
+  // transposed arrays are temporary) and in FP64 only, as adjoint solves are.
+  set_plan_shape(&P->adj_lower, n, P->nnz_U - n, true, false);
+  if (P->lower.line)
+    MTLGPU_TRY(line_plan_detect(ctx, &P->adj_lower, &P->lower, trp, tci));
+  if (P->adj_lower.line)
+    MTLGPU_TRY(line_plan_fill(ctx, &P->adj_lower, 0, trp, tci, tv, P->prec == MTLGPU_FP32));
+  else
+    MTLGPU_TRY(build_sweep_plan(ctx, n, trp, tci, tv, true, false, true, &P->adj_lower));
   MTLGPU_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   dfree(ctx, trp);
   dfree(ctx, tci);
@@ -692,17 +686,17 @@ mtlgpu_status pc_ensure_adjoint(Pc* P) {
   // The reference applies L^T column by column from the last column down
   // (upper_trisolve on the adjoint view, column-major: w[j] -= L[r][j] w[r]
   // for r descending), so each row of L^T takes its entries in descending
-  // column order.
+  // column order.  The grid-line sweeps take a mirrored factor's nearest entry
+  // first, so L^T goes by levels.
   if (n)
     reverse_rows_kernel<<<grid_cap(ctx, n), kBlock, 0, ctx->stream>>>(n, trp, tci, tv);
   MTLGPU_TRY(build_sweep_plan(ctx, n, trp, tci, tv, false, true, false, &P->adj_upper));
-  MTLGPU_TRY(adjoint_line_plan(P, &P->adj_upper, trp, tci, tv));
   MTLGPU_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   dfree(ctx, trp);
   dfree(ctx, tci);
   dfree(ctx, tv);
   if (P->prec == MTLGPU_FP32) {
-    MTLGPU_TRY(sweep_plan_make_fp32(ctx, &P->adj_lower));
+    if (!P->adj_lower.line) MTLGPU_TRY(sweep_plan_make_fp32(ctx, &P->adj_lower));
     MTLGPU_TRY(sweep_plan_make_fp32(ctx, &P->adj_upper));
   }
   MTLGPU_TRY(take_device_error(ctx));
