@@ -361,8 +361,20 @@ mtlgpu_status mtlgpu_pc_set_jacobi_sweeps(mtlgpu_pc* P, int iters);
  * 2 Jacobi iterations (mtlgpu_pc_set_jacobi_sweeps).  A factor with the
  * pattern of a grid stencil is swept along its grid lines, in tiles of lines
  * handed over in shared memory, unless the context was created with
- * MTLGPU_SWEEP=part or =ticket; it reports the kind its levels would choose. */
+ * MTLGPU_SWEEP=part or =ticket; it reports the kind its levels would choose
+ * (mtlgpu_pc_sweep_path tells the sweeps apart). */
 mtlgpu_status mtlgpu_pc_sweep_kind(const mtlgpu_pc* P, int which, int prec, int* kind);
+/* Diagnostics (no counterpart in the reference): the sweep that solves of P run
+ * for factor `which` in precision `prec`: *path = MTLGPU_SWEEP_LEVELS,
+ * MTLGPU_SWEEP_PARTS, MTLGPU_SWEEP_JACOBI or MTLGPU_SWEEP_LINES (along grid
+ * lines). */
+typedef enum {
+  MTLGPU_SWEEP_LEVELS = 0,
+  MTLGPU_SWEEP_PARTS = 1,
+  MTLGPU_SWEEP_JACOBI = 2,
+  MTLGPU_SWEEP_LINES = 3
+} mtlgpu_sweep_kind;
+mtlgpu_status mtlgpu_pc_sweep_path(const mtlgpu_pc* P, int which, int prec, int* path);
 /* Factor sizes and level counts: nnz of the factor as the reference stores it
  * (L of IC(0) includes the diagonal, L of ILU(0) does not). */
 mtlgpu_status mtlgpu_pc_factor_info(const mtlgpu_pc* P, int which, int* nnz, int* n_levels);

@@ -582,22 +582,29 @@ mtlgpu_status mtlgpu_pc_sweep_kind(const mtlgpu_pc* P, int which, int prec, int*
   const int pi = prec == MTLGPU_FP32 ? 1 : 0;
   if (P->jacobi_iters > 0)
     *kind = 2;
-  else if (S.line) {
-    MTLGPU_TRY(pc_ensure_levels(const_cast<mtlgpu_pc*>(P), which));
+  else if (S.line)
     *kind = part_sweep_suits(S) ? 1 : 0;
-  }
   else
     *kind = (S.part && S.part->prec[pi].ready) ? 1 : 0;
+  return MTLGPU_OK;
+}
+
+mtlgpu_status mtlgpu_pc_sweep_path(const mtlgpu_pc* P, int which, int prec, int* path) {
+  if (!P || !path || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0))
+    return MTLGPU_INVALID_ARG;
+  const SweepPlan& S = which == MTLGPU_LOWER ? P->lower : P->upper;
+  const int pi = prec == MTLGPU_FP32 ? 1 : 0;
+  *path = P->jacobi_iters > 0                      ? MTLGPU_SWEEP_JACOBI
+          : S.line                                 ? MTLGPU_SWEEP_LINES
+          : (S.part && S.part->prec[pi].ready)     ? MTLGPU_SWEEP_PARTS
+                                                   : MTLGPU_SWEEP_LEVELS;
   return MTLGPU_OK;
 }
 
 mtlgpu_status mtlgpu_pc_factor_info(const mtlgpu_pc* P, int which, int* nnz, int* n_levels) {
   if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0)) return MTLGPU_INVALID_ARG;
   if (nnz) *nnz = which == MTLGPU_LOWER ? P->nnz_L : P->nnz_U;
-  if (n_levels) {
-    MTLGPU_TRY(pc_ensure_levels(const_cast<mtlgpu_pc*>(P), which));
-    *n_levels = which == MTLGPU_LOWER ? P->lower.n_levels : P->upper.n_levels;
-  }
+  if (n_levels) *n_levels = which == MTLGPU_LOWER ? P->lower.n_levels : P->upper.n_levels;
   return MTLGPU_OK;
 }
 

@@ -949,6 +949,11 @@ mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* P, const SweepPlan* like, co
     return MTLGPU_OK;
   LinePlan* L = new LinePlan();
   P->line = L;
+  // Row t of line j of plane i is of level t + j + i, with three places
+  // t + 2 j + 4 i (a row waits for the next place of the next line of the plane
+  // before).
+  const int step = S.E == 3 ? 2 : 1;
+  P->n_levels = S.B + step * (S.P - 1) + step * step * (S.NI - 1);
   L->shape = S;
   L->args[0] = A[0];
   L->args[1] = A[1];

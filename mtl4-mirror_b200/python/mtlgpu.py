@@ -32,6 +32,7 @@ METHODS = {"cg": CG, "bicgstab": BICGSTAB, "bicg": BICG, "cgs": CGS, "bicgstab_2
            "gmres": GMRES}
 SOLVE_FP64, SOLVE_MIXED = 0, 1
 LOWER, UPPER = 0, 1
+SWEEP_LEVELS, SWEEP_PARTS, SWEEP_JACOBI, SWEEP_LINES = range(4)
 UPDATE_STORE, UPDATE_PLUS, UPDATE_MINUS, UPDATE_TIMES = range(4)
 
 _vp = C.c_void_p
@@ -398,9 +399,16 @@ class Pc:
         check(_lib().mtlgpu_pc_set_jacobi_sweeps(self.h, int(iters)), "pc_set_jacobi_sweeps")
 
     def sweep_kind(self, which, prec=FP64):
-        """0: level-ordered sweep, 1: partitioned sweep, 2: Jacobi iterations."""
+        """0: level-ordered sweep, 1: partitioned sweep, 2: Jacobi iterations; a factor
+        swept along grid lines gives the kind its levels would choose (sweep_path)."""
         k = C.c_int()
         check(_lib().mtlgpu_pc_sweep_kind(self.h, which, prec, C.byref(k)), "pc_sweep_kind")
+        return k.value
+
+    def sweep_path(self, which, prec=FP64):
+        """The sweep that runs: SWEEP_LEVELS, SWEEP_PARTS, SWEEP_JACOBI or SWEEP_LINES."""
+        k = C.c_int()
+        check(_lib().mtlgpu_pc_sweep_path(self.h, which, prec, C.byref(k)), "pc_sweep_path")
         return k.value
 
     def factor_info(self, which):
