@@ -69,6 +69,28 @@ struct GridRow {
     }
     at = (long long)(row / kGridSlice) * (W ? W : A.W) * kGridSlice + row % kGridSlice;
   }
+  // Entries k0 to k0 + C - 1 of an inner row, for W = 0.  Chunks of 8 and what is
+  // left in one of its own length: with the last offset repeated up to 8 (a
+  // tridiagonal matrix issued 16 loads per row for 6) these matrices were slower
+  // than on SELL-32; with a predicate per load the FP64 kernels spilled.  n = 2M, us,
+  // SELL-32 / repeated / now: 3 offsets FP64 product 22.0 / 24.6 / 18.5, FP32 17.4 / 25.4 /
+  // 14.9, FP32 apply 25.9 / 41.1 / 25.3, a mixed CG iteration 66 / 92 / 57; 6: FP64 23.1 /
+  // 26.7 / 24.6, FP32 20.5 / 26.0 / 18.4; 11: 40.5 / 41.2 / 38.9, 35.0 / 39.9 / 24.6, 41.0 /
+  // 44.9 / 32.1, 110 / 110 / 77; 19: 67.1 / 61.2 / 59.4, 51.2 / 55.3 / 35.2, 68.4 / 65.9 / 42.3,
+  // 165 / 160 / 111; 31: 104.5 / 87.9 / 86.0, 77.9 / 71.4 / 53.2, 86.3 / 69.8 / 61.0, 228 / 176 / 147.
+  template <int C, typename Get, typename Fold>
+  __device__ __forceinline__ void part(const T* __restrict__ vp, int k0, Get get, Fold fold) const {
+    T a[C];
+    decltype(get(0)) g[C];
+#pragma unroll
+    for (int u = 0; u < C; u++) {
+      a[u] = __ldlu(vp + (k0 + u) * kGridSlice);
+      g[u] = get(row + A.off[k0 + u]);
+    }
+#pragma unroll
+    for (int u = 0; u < C; u++)
+      if (mask >> (k0 + u) & 1u) fold(a[u], g[u]);
+  }
   // fold(a, g) over the row's entries in ascending offset, g = get(c) at the
   // entry's column c; C entries' loads are issued before the first is used.
   template <int C, typename Get, typename Fold>
@@ -91,18 +113,17 @@ struct GridRow {
             if (k0 + u < W && (mask >> (k0 + u) & 1u)) fold(a[u], g[u]);
         }
       } else {
-        for (int k0 = 0; k0 < A.W; k0 += C) {
-          T a[C];
-          decltype(get(0)) g[C];
-#pragma unroll
-          for (int u = 0; u < C; u++) {  // past the last offset: the last one again
-            const int k = min(k0 + u, A.W - 1);
-            a[u] = __ldlu(vp + k * kGridSlice);
-            g[u] = get(row + A.off[k]);
-          }
-#pragma unroll
-          for (int u = 0; u < C; u++)
-            if (k0 + u < A.W && (mask >> (k0 + u) & 1u)) fold(a[u], g[u]);
+        static_assert(W || C == 8, "a remainder of 1 to 7");
+        int k0 = 0;
+        for (; k0 + C <= A.W; k0 += C) part<C>(vp, k0, get, fold);
+        switch (A.W - k0) {  // the same for every thread
+          case 1: part<1>(vp, k0, get, fold); break;
+          case 2: part<2>(vp, k0, get, fold); break;
+          case 3: part<3>(vp, k0, get, fold); break;
+          case 4: part<4>(vp, k0, get, fold); break;
+          case 5: part<5>(vp, k0, get, fold); break;
+          case 6: part<6>(vp, k0, get, fold); break;
+          case 7: part<7>(vp, k0, get, fold); break;
         }
       }
     } else {
