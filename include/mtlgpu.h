@@ -249,6 +249,15 @@ mtlgpu_status mtlgpu_csr_values_grad(mtlgpu_csr* A, const double* d_lambda, cons
  * *h_choice (when non-NULL) receives 2 (SELL-32 or grid) or 0 (CSR-stream).  No
  * counterpart in the reference (the layout behind mat_vec_mult.hpp:620-689). */
 mtlgpu_status mtlgpu_csr_autotune(mtlgpu_csr* A, int* h_choice);
+/* Diagnostics (no counterpart in the reference): the layout A's products read:
+ * *layout = MTLGPU_LAYOUT_STREAM, MTLGPU_LAYOUT_SELL or MTLGPU_LAYOUT_GRID (at
+ * most 32 distinct offsets column - row, values by offset). */
+typedef enum {
+  MTLGPU_LAYOUT_STREAM = 0,
+  MTLGPU_LAYOUT_SELL = 1,
+  MTLGPU_LAYOUT_GRID = 2
+} mtlgpu_layout;
+mtlgpu_status mtlgpu_csr_layout(const mtlgpu_csr* A, int* layout);
 
 /* y = alpha * A * x + beta * y.  With (alpha, beta) = (1, 0), (1, 1), (-1, 1)
  * this is y = A*x, y += A*x, y -= A*x (mtl/operation/mult.hpp:43-70,
@@ -270,7 +279,7 @@ mtlgpu_status mtlgpu_spmv_transposed(mtlgpu_csr* A, const double* d_x, double* d
  * fused_expr.hpp:57-77); it is the product kernel of the device CG with
  * Jacobi-applied factors.  prec MTLGPU_FP32 (float vectors, A's values
  * rounded to float) or MTLGPU_FP64.  p_out must differ from z and p.  Needs
- * the SELL-32 layout (MTLGPU_NOT_SUPPORTED otherwise).  Asynchronous on the
+ * the SELL-32 or grid layout (MTLGPU_NOT_SUPPORTED otherwise).  Asynchronous on the
  * context's stream. */
 mtlgpu_status mtlgpu_cg_direction_product(mtlgpu_csr* A, int prec, const void* d_z, double beta,
                                           const void* d_p, void* d_p_out, void* d_q,

@@ -708,6 +708,14 @@ mtlgpu_status mtlgpu_solve_host(int method, mtlgpu_csr* A, mtlgpu_pc* P, double*
   return s;
 }
 
+mtlgpu_status mtlgpu_csr_layout(const mtlgpu_csr* A, int* layout) {
+  if (!A || !layout) return MTLGPU_INVALID_ARG;
+  *layout = A->spmv_kernel != 2 ? MTLGPU_LAYOUT_STREAM
+            : A->sell.grid      ? MTLGPU_LAYOUT_GRID
+                                : MTLGPU_LAYOUT_SELL;
+  return MTLGPU_OK;
+}
+
 mtlgpu_status mtlgpu_csr_autotune(mtlgpu_csr* A, int* choice) {
   if (!A) return MTLGPU_INVALID_ARG;
   int c = 0;

@@ -33,6 +33,7 @@ METHODS = {"cg": CG, "bicgstab": BICGSTAB, "bicg": BICG, "cgs": CGS, "bicgstab_2
 SOLVE_FP64, SOLVE_MIXED = 0, 1
 LOWER, UPPER = 0, 1
 SWEEP_LEVELS, SWEEP_PARTS, SWEEP_JACOBI, SWEEP_LINES = range(4)
+LAYOUT_STREAM, LAYOUT_SELL, LAYOUT_GRID = range(3)
 UPDATE_STORE, UPDATE_PLUS, UPDATE_MINUS, UPDATE_TIMES = range(4)
 
 _vp = C.c_void_p
@@ -350,6 +351,12 @@ class Csr:
         c = C.c_int()
         check(_lib().mtlgpu_csr_autotune(self.h, C.byref(c)), "autotune")
         return c.value
+
+    def layout(self):
+        """What the products read: LAYOUT_STREAM, LAYOUT_SELL or LAYOUT_GRID."""
+        k = C.c_int()
+        check(_lib().mtlgpu_csr_layout(self.h, C.byref(k)), "csr_layout")
+        return k.value
 
     def close(self):
         if self.h:

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from test_gpu_grid_layout import offsets_matrix
+from test_gpu_layout_choice import expected
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,23 @@ def test_width(M, restate, monkeypatch, W):
             assert np.array_equal(g, i), j
         else:
             assert np.linalg.norm(g - i) <= 1e-8 * np.linalg.norm(i), j
+
+
+@pytest.mark.parametrize("n", [8, 31, 32, 33, 64, 127, 128, 129, 160, 255, 256, 257, 383, 384,
+                               385, 1000])
+@pytest.mark.parametrize("offs", [[0], [0, 1], [-2, 0], [0, 1, -1], [0, 1, -1, 2, -2]])
+def test_row_counts(M, ctx, restate, n, offs):
+    # around warps and slices of 128 rows; a vector off the 16-byte grid
+    A = offsets_matrix(n, offs, 0.0, n)
+    dA = M.Csr(ctx, *A[1:])
+    assert dA.layout() == expected(M, A)
+    x = M.uniform(n, 3)
+    for shift in (0, 1):
+        a, y = ctx.to_device(np.concatenate([np.zeros(shift), x])), ctx.array(n + shift)
+
+        class View:
+            def __init__(self, v):
+                self.n, self.ptr = n, M.C.c_void_p(v.ptr.value + 8 * shift)
+        dA.spmv(View(a), View(y))
+        assert np.array_equal(y.download()[shift:], restate.spmv(A, x))
+    dA.close()
