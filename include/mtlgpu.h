@@ -472,7 +472,8 @@ mtlgpu_status mtlgpu_solve_batched(int method, mtlgpu_csr* A, mtlgpu_pc* P, int 
  * also 512 and 1024), and the row count below which a system is solved by a
  * single CTA (0, 8192, 32768), and keeps the fastest on A in place of the
  * shape that follows from the systems' sizes.
- * *h_choice = 1000 * rows + 100 * CTAs + lanes.  Applies to the persistent-launch path
+ * *h_choice = 1000 * rows + 100 * CTAs + lanes; mtlgpu_batched_shape gives the
+ * threads per CTA too.  Applies to the persistent-launch path
  * (P NULL, diagonal, or factors applied by Jacobi iterations); other
  * preconditioners return MTLGPU_NOT_SUPPORTED.  No counterpart in the
  * reference. */
@@ -480,6 +481,12 @@ mtlgpu_status mtlgpu_batched_autotune(mtlgpu_csr* A, mtlgpu_pc* P, int count,
                                       const int32_t* h_offsets, const double* d_x,
                                       const double* d_b, const mtlgpu_iter_params* params,
                                       int* h_choice);
+/* The shape kept by mtlgpu_batched_autotune: CTAs per large system, lanes per row,
+ * threads per CTA and the rows below which one CTA solves a system
+ * (MTLGPU_BATCH_SHAPE="ctas,lanes,rows,threads" asks for the same shape); all 0
+ * while the shape follows from the systems' sizes.  Any pointer may be NULL. */
+mtlgpu_status mtlgpu_batched_shape(const mtlgpu_csr* A, int* h_ctas, int* h_lanes, int* h_threads,
+                                   int* h_rows);
 
 #if defined(__GNUC__)
 #pragma GCC visibility pop

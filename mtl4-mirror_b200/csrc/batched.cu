@@ -610,3 +610,14 @@ extern "C" mtlgpu_status mtlgpu_solve_batched(int method, mtlgpu_csr* A, mtlgpu_
   if (!A) return MTLGPU_INVALID_ARG;
   return mtlgpu::solve_batched_impl(method, A, P, count, h_offsets, d_x, d_b, params, h_results);
 }
+
+extern "C" mtlgpu_status mtlgpu_batched_shape(const mtlgpu_csr* A, int* h_ctas, int* h_lanes,
+                                              int* h_threads, int* h_rows) {
+  if (!A) return MTLGPU_INVALID_ARG;
+  const mtlgpu::BatchShape none{0, 0, 0, 0}, &s = A->batch.cs ? A->batch : none;
+  if (h_ctas) *h_ctas = s.cs;
+  if (h_lanes) *h_lanes = s.g;
+  if (h_threads) *h_threads = s.threads;
+  if (h_rows) *h_rows = s.small_rows;
+  return MTLGPU_OK;
+}

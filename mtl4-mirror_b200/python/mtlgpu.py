@@ -512,6 +512,13 @@ def batched_autotune(A, P, offsets, x, b, **kw):
     return c.value
 
 
+def batched_shape(A):
+    """The shape batched_autotune kept on A: (CTAs, lanes, threads, rows), zeros when none."""
+    q = [C.c_int() for _ in range(4)]
+    check(_lib().mtlgpu_batched_shape(A.h, *(C.byref(k) for k in q)), "batched_shape")
+    return tuple(k.value for k in q)
+
+
 def solve_host(method, A, P, x, b, **kw):
     """Same with host numpy x (updated in place) and b."""
     hist = np.zeros(2 * kw.get("max_iter", 1000) + 8)
