@@ -28,6 +28,7 @@ struct Ctx {
   bool own_stream = false;
   long long spin_limit = 1ll << 26;
   int num_sms = 148;
+  size_t device_bytes = 0;         // memory of the device
   std::string last_error;
   // reduction scratch
   double* d_partials = nullptr;   // kMaxPartials * kPartialWidth
@@ -296,7 +297,7 @@ mtlgpu_status part_sweep_launch(Ctx* ctx, const SweepPlan& S, const T* in, T* ou
                                 const int* skip);
 
 // Sweeps along grid lines (line_sweep.cu), for factors with a grid stencil's
-// pattern.  line_plan_detect and line_plan_fill run outside stream capture;
+// pattern.  line_plan_detect and line_plan_fill run on a stream that is not captured;
 // the records are made before the first exact sweep (pc_ensure_sweeps).
 mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* S, const SweepPlan* like, const int32_t* d_rp,
                                const int32_t* d_ci);
@@ -374,7 +375,7 @@ mtlgpu_status csr_transpose(Ctx* ctx, int n_rows, int n_cols, int nnz, const int
 mtlgpu_status pc_build(Pc* P);
 void pc_release(Pc* P);
 mtlgpu_status pc_ensure_adjoint(Pc* P);
-mtlgpu_status pc_ensure_sweeps(Pc* P, int prec);    // exact sweeps ready (before any capture)
+mtlgpu_status pc_ensure_sweeps(Pc* P, int prec);    // exact sweeps ready
 mtlgpu_status pc_ensure_levels(Pc* P, int which);
 template <typename T>
 mtlgpu_status pc_apply_t(Pc* P, const T* r, T* z, bool adjoint, const int* skip,

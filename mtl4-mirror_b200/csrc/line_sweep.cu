@@ -804,12 +804,12 @@ bool line_layout_t(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
 size_t record_bytes(const LineArgs& A) {
   return (size_t)A.ntiles * A.compute_warps * A.blocks * A.stage;
 }
-bool line_layout(Ctx* ctx, const LineShape& L, int ts, size_t device, LineArgs* A) {
+bool line_layout(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
   const bool fits =
       L.E == 1 ? (L.G == 1 ? line_layout_t<1, 1>(ctx, L, ts, A) : line_layout_t<2, 1>(ctx, L, ts, A))
                : (L.G == 1 ? line_layout_t<1, 3>(ctx, L, ts, A) : line_layout_t<4, 3>(ctx, L, ts, A));
   return fits && line_records_fit((long long)L.n * A->rec_bytes, (long long)record_bytes(*A),
-                                  (long long)device);
+                                  (long long)ctx->device_bytes);
 }
 
 template <typename T>
@@ -943,10 +943,7 @@ mtlgpu_status line_plan_detect(Ctx* ctx, SweepPlan* P, const SweepPlan* like, co
   dfree(ctx, d_s);
   MTLGPU_TRY(st);
   LineArgs A[2];
-  size_t free_bytes = 0, device = 0;
-  MTLGPU_TRY_CUDA(ctx, cudaMemGetInfo(&free_bytes, &device));
-  if (!found || !line_layout(ctx, S, 8, device, &A[0]) || !line_layout(ctx, S, 4, device, &A[1]))
-    return MTLGPU_OK;
+  if (!found || !line_layout(ctx, S, 8, &A[0]) || !line_layout(ctx, S, 4, &A[1])) return MTLGPU_OK;
   LinePlan* L = new LinePlan();
   P->line = L;
   // Row t of line j of plane i is of level t + j + i, with three places
