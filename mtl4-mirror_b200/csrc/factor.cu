@@ -587,14 +587,7 @@ mtlgpu_status build_ilu0(Pc* P) {
 
 }  // namespace
 
-// The exact sweeps of P in precision `prec` ready to launch: for grid-line
-// plans the records, made at the first exact solve (factors applied by Jacobi
-// iterations alone never need them).  FP32 records are made with the
-// preconditioner: mtlgpu_pc_apply_f32 does not wait for the stream, so its first
-// call may be inside a capture, where nothing can be allocated.  Call before any
-// stream capture.
-mtlgpu_status pc_ensure_sweeps(Pc* P, int prec) {
-  if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0)) return MTLGPU_OK;
+static mtlgpu_status fill_line_records(Pc* P, int prec) {
   Ctx* ctx = P->A->ctx;
   const bool round = P->prec == MTLGPU_FP32;
   if (P->lower.line && !line_records_ready(P->lower, prec))
@@ -602,6 +595,39 @@ mtlgpu_status pc_ensure_sweeps(Pc* P, int prec) {
   if (P->upper.line && !line_records_ready(P->upper, prec))
     MTLGPU_TRY(line_plan_fill(ctx, &P->upper, prec, P->d_Urp, P->d_Uci, P->d_Uv, round));
   return MTLGPU_OK;
+}
+
+// The exact sweeps of P in precision `prec` ready to launch: for grid-line
+// plans the records, made at the first exact solve (factors applied by Jacobi
+// iterations alone never need them).  mtlgpu_pc_apply_f32 does not wait for the
+// stream, so its first call may be inside a capture of the caller's, and memory
+// allocated there would be the graph's: the records are then made on a stream of
+// their own (the factors were final when the preconditioner was created).  The
+// library's own captures call this before they begin.
+mtlgpu_status pc_ensure_sweeps(Pc* P, int prec) {
+  if (!P || (P->kind != MTLGPU_PC_IC0 && P->kind != MTLGPU_PC_ILU0)) return MTLGPU_OK;
+  if ((!P->lower.line || line_records_ready(P->lower, prec)) &&
+      (!P->upper.line || line_records_ready(P->upper, prec)))
+    return MTLGPU_OK;
+  Ctx* ctx = P->A->ctx;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
+  if (capture == cudaStreamCaptureStatusNone) return fill_line_records(P, prec);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  MTLGPU_TRY_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+  const cudaStream_t captured = ctx->stream;
+  cudaStream_t side = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+  mtlgpu_status st = MTLGPU_OK;
+  if (e == cudaSuccess) {
+    ctx->stream = side;
+    st = fill_line_records(P, prec);
+    ctx->stream = captured;
+    e = cudaStreamSynchronize(side);
+    cudaStreamDestroy(side);
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return e == cudaSuccess ? st : set_cuda_error(ctx, e, "records of a captured sweep");
 }
 
 // Levels of a factor that was set up without them.
@@ -651,7 +677,6 @@ mtlgpu_status pc_build(Pc* P) {
   const bool f32 = P->prec == MTLGPU_FP32;
   MTLGPU_TRY(part_plan_build(ctx, &P->lower, f32));
   MTLGPU_TRY(part_plan_build(ctx, &P->upper, f32));
-  if (f32) MTLGPU_TRY(pc_ensure_sweeps(P, MTLGPU_FP32));
   return take_device_error(ctx);
 }
 
