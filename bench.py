@@ -135,10 +135,15 @@ def layout_bytes(rp, ci):
     Jacobi applies read, beside the values and vectors: the grid layout (a mask
     of 1, 2 or 4 bytes per row, nothing per entry) where the matrix has at most
     32 offsets and padding every row to all of them adds at most a quarter;
-    else SELL-32 (sell_index_bytes and a 4-byte offset per 32 rows)."""
+    else SELL-32 (sell_index_bytes and a 4-byte offset per 32 rows).  Products of
+    a matrix where padding rows to the longest of their 32 adds more than a
+    fifth read CSR: a 4-byte index per entry and a 4-byte start per row."""
     n = len(rp) - 1
+    ln = np.diff(rp)
+    if np.pad(ln, (0, -n % 32)).reshape(-1, 32).max(1, initial=0).sum() * 32 > 1.2 * len(ci):
+        return 4, 4
     if os.environ.get("MTLGPU_SELL_INDEX", "") != "32" and len(ci):
-        rows = np.repeat(np.arange(n, dtype=np.int64), np.diff(rp))
+        rows = np.repeat(np.arange(n, dtype=np.int64), ln)
         w = len(np.unique(ci - rows))
         if w <= 32 and w * n <= 1.25 * len(ci):
             return 0, 1 if w <= 8 else 2 if w <= 16 else 4

@@ -749,8 +749,10 @@ void batch_work_free(Ctx* ctx, BatchWork* w) {
 // 1,000-65,536 rows 8.1 / 5.7 / 6.7 (16.3), 32 of them 7.1 / 5.0 / 4.4 (13.1), 16 of
 // 20,000 rows 3.3 / 2.4 / 2.1 (5.5), 300 of 8,000 6.1 / 7.0 / 9.4 (6.9), 1,024 of
 // 3,000 6.7 / 7.1 / 8.4 (7.5).  Solved by one CTA below 4,096 / 2,048 / 1,024 rows:
-// the 96 systems 6.2 / 5.7 / 5.5 (512 threads), the 1,024 systems 6.7 / 8.5 / 8.5 (256);
-// 100 systems of 1,500 rows 1.9 / 1.9 / 0.76 (their share is 1,516 threads).
+// with 256 threads the 1,024 systems 6.7 / 8.5 / 8.5; with 512 three draws of the 96 to
+// 64 systems 5.7 / 5.5 / 5.3, 5.6 / 5.5 / 5.6 and 4.7 / 4.6 / 4.7, and 40 of them with 400 of
+// 1,500 rows 5.3 / 5.3 / 6.4: hence 2,048.  100 systems of 1,500 rows 1.9 / 1.9 / 0.76
+// (their share is 1,516 threads).
 // The stream product takes the rows of a warp together: 3-10 % faster than 8
 // lanes per row here, but one lane adds up a row, so only for rows that fit its
 // chunk of 256 entries.

@@ -462,7 +462,11 @@ __global__ void __launch_bounds__(kBlock, grid_blocks_t<T>())
 // launch it saves (~2 us) weighs less.  One iteration, K_C / split, us (FP64; FP32
 // of the mixed solve): 7-point 64^3 24.8 / 25.6; 23.4 / 25.7, 96^3 46.9 / 45.6;
 // 38.4 / 38.0, 128^3 96.0 / 91.6; 68.3 / 66.0, 144^3 135.8 / 126.1; 91.7 / 86.5; 5-point
-// 1024^2 44.0 / 44.4; 37.0 / 36.5, 1400^2 77.4 / 76.2; 57.8 / 54.9.
+// 800^2 31.9 / 32.5; 28.8 / 29.0, 1024^2 44.0 / 44.4; 37.0 / 36.5, 1400^2 77.4 / 76.2;
+// 57.8 / 54.9; 27-point 64^3 40.5 / 42.4; 32.3 / 32.5, 96^3 98.8 / 98.5; 63.0 / 62.3, 104^3
+// 124.0 / 121.9; 75.8 / 72.7, 128^3 220.6 / 215.5; 137.9 / 135.5.  The two meet between
+// 0.8 and 1.1 million rows by stencil and type; one line for all costs 1 % at
+// 1024^2 in FP64 and forgoes 3 % at 96^3.
 bool direction_split(const Sell& S) { return S.grid && S.n >= 1 << 20; }
 
 struct BetaSrc {

@@ -404,7 +404,8 @@ mtlgpu_status csr_analyse(Csr* A) {
   A->max_row = (int)h_stats[0];
   A->mean_row = A->n_rows ? double(h_stats[1]) / A->n_rows : 0.0;
 
-  // SpMV layout.  SELL-32 where its padding is small (stencils: < 1 %);
+  // SpMV layout.  The grid layout or SELL-32 (sell_build chooses) where padding
+  // rows to their slice's longest adds at most a fifth (kSellMaxPadding);
   // otherwise CSR-stream row blocks (greedy: up to 32 rows and 32*kStreamK
   // entries; a longer row forms a block of its own).
   {
