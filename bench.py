@@ -644,7 +644,7 @@ def adjoint_workload(M, ctx, stream):
 
 def profile_case(case, grid, launches):
     """Runs one kernel (or one solve) of the path a few times on an N^3
-    Laplacian, for profiler captures: 'spmv' (FP64 y = A x, SELL-32),
+    Laplacian, for profiler captures: 'spmv' (FP64 y = A x),
     'spmv32' (FP32), 'jacobi32' (FP32 IC(0) apply with JACOBI_K Jacobi
     iterations per triangle), 'sweep64' / 'sweep32' (exact IC(0) lower sweep),
     'mixed' (complete mixed solves of the headline configuration, for the
