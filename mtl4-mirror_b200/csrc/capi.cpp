@@ -49,8 +49,6 @@ mtlgpu_status set_device(Ctx* ctx) {
 mtlgpu_status ctx_init(Ctx* ctx) {
   MTLGPU_TRY_CUDA(ctx, cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount,
                                               ctx->device));
-  size_t free_bytes = 0;
-  MTLGPU_TRY_CUDA(ctx, cudaMemGetInfo(&free_bytes, &ctx->device_bytes));
   if (const char* m = std::getenv("MTLGPU_SWEEP_BLOCKS_PER_SM")) ctx->sweep_blocks_per_sm = std::atoi(m);
   if (const char* m = std::getenv("MTLGPU_SWEEP")) {
     if (!std::strcmp(m, "part")) ctx->part_sweeps = 1;

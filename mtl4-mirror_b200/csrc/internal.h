@@ -28,7 +28,7 @@ struct Ctx {
   bool own_stream = false;
   long long spin_limit = 1ll << 26;
   int num_sms = 148;
-  size_t device_bytes = 0;         // memory of the device
+  size_t device_bytes = 0;         // memory of the device, once asked for
   std::string last_error;
   // reduction scratch
   double* d_partials = nullptr;   // kMaxPartials * kPartialWidth

@@ -808,8 +808,14 @@ bool line_layout(Ctx* ctx, const LineShape& L, int ts, LineArgs* A) {
   const bool fits =
       L.E == 1 ? (L.G == 1 ? line_layout_t<1, 1>(ctx, L, ts, A) : line_layout_t<2, 1>(ctx, L, ts, A))
                : (L.G == 1 ? line_layout_t<1, 3>(ctx, L, ts, A) : line_layout_t<4, 3>(ctx, L, ts, A));
-  return fits && line_records_fit((long long)L.n * A->rec_bytes, (long long)record_bytes(*A),
-                                  (long long)ctx->device_bytes);
+  if (!fits) return false;
+  const long long own = (long long)L.n * A->rec_bytes, padded = (long long)record_bytes(*A);
+  if (line_records_fit(own, padded, 0)) return true;
+  size_t free_bytes = 0;  // asking for the device's memory takes up to milliseconds
+  if (!ctx->device_bytes &&
+      cudaMemGetInfo(&free_bytes, &ctx->device_bytes) != cudaSuccess)
+    cudaGetLastError();
+  return line_records_fit(own, padded, (long long)ctx->device_bytes);
 }
 
 template <typename T>
