@@ -566,14 +566,17 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     for (; blk < A.steps / KL; blk++) {
       const int st = blk & smask, s0 = blk * KL;
       long long polls = 0;
-      while (s0 + KL - ld_shared_acquire(prog + cw * 4) > A.stages * KL) {
+      int at;  // the compute warp's step; kNever here: it gave up
+      while (s0 + KL - (at = ld_shared_acquire(prog + cw * 4)) > A.stages * KL) {
         if (++polls >= limit || *(volatile int*)&s_done == A.compute_warps) {
           stop = true;
           break;
         }
         __nanosleep(20);
       }
-      if (__any_sync(0xffffffffu, stop)) break;
+      // A stage is filled again only once the warp has taken it: its barrier must
+      // have completed the phase before.
+      if (__any_sync(0xffffffffu, stop || at >= kNever)) break;
       if (lane == 0) {
         if ((unsigned)(blk - b0) < (unsigned)A.blocks) {
           mbar_arrive_expect_tx(bar + st, kStage);
@@ -590,10 +593,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       __syncwarp();
       mbar_arrive_cp_async(bar + st);
     }
-    // every copy has landed before the block ends (also one that gave up)
+    // Every copy has landed before the block ends, also one that gave up: copies
+    // wait for nobody, so this has a bound of its own.
     cp_async_wait_all();
+    const long long drain = limit > (1ll << 24) ? limit : (1ll << 24);
     for (int k = max(0, blk - A.stages); k < blk; k++)
-      mbar_wait(bar + (k & smask), (unsigned)(k / A.stages) & 1u, limit);
+      mbar_wait(bar + (k & smask), (unsigned)(k / A.stages) & 1u, drain);
   }
   __syncthreads();
   if (tid == 0) {
